@@ -44,6 +44,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 def lib():
@@ -66,6 +67,32 @@ def lib():
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+def host():
+    """The compiled host side (``_host.so``), bound to the loaded library.
+
+    Its functions do the checks, output tensors and launch of an entry point's common case in C++ and return ``None``
+    for a call they leave to the Python code. Like the library it has no fallback: a missing file raises.
+    """
+    global _host
+    if _host is None:
+        handle = lib()
+        try:
+            from . import _host as module
+        except ImportError as err:
+            raise RuntimeError(
+                f"warpy_kernels_b200/_host.so is missing or does not load ({err}): build it with "
+                f"`make -C {os.path.join(_HERE, 'csrc')}`"
+            ) from err
+        module.bind({name: address(getattr(handle, name)) for name in SIGNATURES})
+        _host = module
+    return _host
+
+
+def address(fn):
+    """Address of a function of the library, as ``_host.launch`` takes it."""
+    return ctypes.cast(fn, _ptr).value
 
 
 def stream_ptr(device=None):

@@ -150,20 +150,25 @@ def make_attn_bwd(
     args.lse_strides = (ctypes.c_int64 * 2)(*lsev.stride()[:2])
     args.B, args.Hq, args.Hkv, args.Nq, args.Nk, args.d = B, Hq, Hkv, Nq, Nk, d
     args.causal, args.softmax_scale = int(bool(causal)), float(softmax_scale)
-    keep = (qv, kv, vv, ov, dov, lsev, dq_, dk_, dv_, workspace, dq, dk, dv)  # inputs, scratch and outputs
+    keep = (qv, kv, vv, ov, dov, lsev, dq_, dk_, dv_, workspace, dq, dk, dv, args)  # inputs, scratch and outputs
 
-    entry = lib.wk_attn_bwd_bf16 if bf16 else lib.wk_attn_bwd_fp8
+    host = _lib.host()
+    entry = _lib.address(lib.wk_attn_bwd_bf16 if bf16 else lib.wk_attn_bwd_fp8)
+    block, index = ctypes.addressof(args), dev.index
 
     def launch():
-        with torch.cuda.device(dev):
-            code = entry(ctypes.byref(args), _lib.stream_ptr(dev))
-        _lib.check(code, "attn_bwd")
+        _lib.check(host.launch(entry, block, index), "attn_bwd")
         return keep
 
     def finish():
         return dq, dk, dv
 
     return launch, finish
+
+
+def common_case(*args, **config):
+    """The whole call in compiled code, or ``None`` if it needs a copy, is invalid or not plain."""
+    return _lib.host().attn_bwd(*args, **config)
 
 
 def attn_bwd(
@@ -175,9 +180,11 @@ def attn_bwd(
     Returns:
         ``(dq, dk, dv)`` in bf16.
     """
-    launch, finish = make_attn_bwd(
-        q, k, v, out, lse, pmax, dout, q_descale, k_descale, v_descale, causal, softmax_scale, **config
-    )
+    args = (q, k, v, out, lse, pmax, dout, q_descale, k_descale, v_descale, causal, softmax_scale)
+    done = common_case(*args, **config)
+    if done is not None:
+        return done
+    launch, finish = make_attn_bwd(*args, **config)
     launch()
     return finish()
 

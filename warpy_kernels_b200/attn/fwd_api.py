@@ -12,7 +12,7 @@ import torch
 
 from .. import _lib
 from ..arch import require
-from ..utils import autotune, cached_tensor, check_descale, round_up, tune_key, tune_lookup
+from ..utils import any_tuned, autotune, cached_tensor, check_descale, round_up, tune_key, tune_lookup
 
 BM = 128
 
@@ -32,20 +32,13 @@ class _FwdArgs(ctypes.Structure):
     ]
 
 
-_flag_buffers = {}
-
-
 def _block_flags(dev, nbytes):
     """Zeroed flag scratch of the forward for the current stream of ``dev``, at least ``nbytes`` long.
 
     The kernels mark query blocks whose scores outgrow the range of their fixed row reference; the library
     recomputes those and hands the buffer back all zero, so calls that follow one another on a stream can share it.
     """
-    key = (dev, torch.cuda.current_stream(dev).cuda_stream)
-    buf = _flag_buffers.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = _flag_buffers[key] = torch.zeros(max(nbytes, 1 << 16), dtype=torch.uint8, device=dev)
-    return buf
+    return _lib.host().block_flags(dev.index, nbytes)
 
 
 def _kernel_view(x):
@@ -209,14 +202,14 @@ def make_attn_fwd(
     # closure and drop the tensors it was handed
     keep = (qv, kv, vv, dq_, dk_, dv_, seq, out_k, out, lse, pmax)
     lib = _lib.lib()
-    entry = lib.wk_attn_fwd_bf16 if bf16 else lib.wk_attn_fwd_fp8
+    host = _lib.host()
+    entry = _lib.address(lib.wk_attn_fwd_bf16 if bf16 else lib.wk_attn_fwd_fp8)
+    block, index = ctypes.addressof(args), dev.index
     args.workspace_bytes = lib.wk_attn_fwd_workspace_bytes(B, Hq, Nq)
 
     def launch():
-        with torch.cuda.device(dev):
-            args.workspace = _block_flags(dev, args.workspace_bytes).data_ptr()
-            code = entry(ctypes.byref(args), _lib.stream_ptr(dev))
-        _lib.check(code, "attn_fwd")
+        args.workspace = host.block_flags(index, args.workspace_bytes).data_ptr()
+        _lib.check(host.launch(entry, block, index), "attn_fwd")
         if not out_direct:
             out.copy_(out_k)
         return keep
@@ -226,12 +219,23 @@ def make_attn_fwd(
     return launch, out, None, None
 
 
+def common_case(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config):
+    """The whole call in compiled code, or ``None`` if it needs a copy, is invalid or not plain."""
+    if any_tuned() and config.get("ctas_per_sm") is None and q.dtype == torch.float8_e4m3fn and q.dim() == k.dim() == 4:
+        tuned = tune_lookup(tune_key("fwd", q.shape[3], causal, q.shape[2], k.shape[2], q.shape[1] // k.shape[1]))
+        config["ctas_per_sm"] = (tuned or {}).get("ctas_per_sm")
+    return _lib.host().attn_fwd(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config)
+
+
 def attn_fwd(q, k, v, q_descale=None, k_descale=None, v_descale=None, causal=False, softmax_scale=None, **config):
     """Run the attention forward kernel; arguments as in ``make_attn_fwd``.
 
     Returns:
         ``(out, lse, pmax)``.
     """
+    done = common_case(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config)
+    if done is not None:
+        return done
     launch, out, lse, pmax = make_attn_fwd(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config)
     launch()
     return out, lse, pmax

@@ -13,7 +13,7 @@ import torch
 
 from .. import _lib
 from ..arch import require
-from ..utils import gemm_tune_key, time_candidates, tune_lookup, tune_store
+from ..utils import any_tuned, gemm_tune_key, time_candidates, tune_lookup, tune_store
 
 _TYPES = {torch.bfloat16: "bf16", torch.float16: "f16"}
 BM = 128
@@ -242,13 +242,9 @@ def make_gemm(
         args.cta_pair = 0 if cta_pair is None else 1 if cta_pair else 2
         args.group_m = int(group_m or 0)
         fill_epilogue(args)
-        keep = (a, b, out, scale_a, scale_b, pre_out, pre_in, q_mx, s_mx)  # inputs and outputs stay alive
+        keep = (a, b, out, scale_a, scale_b, pre_out, pre_in, q_mx, s_mx, args)  # inputs and outputs stay alive
 
-        def launch():
-            with torch.cuda.device(dev):
-                code = lib.wk_gemm_16bit(ctypes.byref(args), _lib.stream_ptr(dev))
-            _lib.check(code, "gemm (16-bit)")
-            return keep
+        what, entry = "gemm (16-bit)", _lib.address(lib.wk_gemm_16bit)
 
     else:
         ws_bytes = lib.wk_gemm_mxfp8_workspace_bytes(m, n, k)
@@ -270,16 +266,27 @@ def make_gemm(
         args.cta_pair = 0 if cta_pair is None else 1 if cta_pair else 2
         args.group_m = int(group_m or 0)
         fill_epilogue(args)
-        keep = (a, b, out, a_scale_mx, b_tiled, scale_a, scale_b, workspace, pre_out, pre_in, q_mx, s_mx)
+        keep = (a, b, out, a_scale_mx, b_tiled, scale_a, scale_b, workspace, pre_out, pre_in, q_mx, s_mx, args)
 
-        def launch():
-            with torch.cuda.device(dev):
-                code = lib.wk_gemm_mxfp8(ctypes.byref(args), _lib.stream_ptr(dev))
-            _lib.check(code, "gemm (fp8)")
-            return keep
+        what, entry = "gemm (fp8)", _lib.address(lib.wk_gemm_mxfp8)
+
+    host, block, index = _lib.host(), ctypes.addressof(args), dev.index
+
+    def launch():
+        _lib.check(host.launch(entry, block, index), what)
+        return keep
 
     mx = (q_mx, s_mx) if out_mx else ()
     return (launch, out, pre_out, *mx) if act == "gelu" else (launch, out, *mx)
+
+
+def _tuned(a, b, kwargs):
+    """What ``autotune_gemm`` stored for the shape of these operands, or an empty dict."""
+    if a.dim() != 2 or b.dim() != 2:
+        return {}
+    m, k = a.shape[::-1] if kwargs.get("a_trans") else a.shape
+    n = b.shape[1] if kwargs.get("b_trans") else b.shape[0]
+    return tune_lookup(gemm_tune_key("gemm_fp8" if a.dtype == torch.float8_e4m3fn else "gemm", m, n, k)) or {}
 
 
 def gemm(a, b, out=None, **kwargs):
@@ -289,6 +296,13 @@ def gemm(a, b, out=None, **kwargs):
         ``[M, N]`` in the output dtype, or ``(out, pre)`` if ``act="gelu"``. With ``out_mx``, a tuple that ends with
         the e4m3 values and their scales.
     """
+    options = kwargs
+    if any_tuned() and (kwargs.get("cta_pair") is None or kwargs.get("group_m") is None):
+        tuned = _tuned(a, b, kwargs)
+        options = dict(kwargs, **{key: tuned.get(key) for key in ("cta_pair", "group_m") if kwargs.get(key) is None})
+    done = _lib.host().gemm(a, b, out, **options)
+    if done is not None:
+        return done
     launch, out, *rest = make_gemm(a, b, out, **kwargs)
     launch()
     return (out, *rest) if kwargs.get("act") == "gelu" or kwargs.get("out_mx") else out

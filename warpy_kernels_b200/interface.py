@@ -3,6 +3,7 @@
 import torch
 
 from .arch import require
+from .attn import bwd_api, fwd_api
 from .gemm.api import autotune_gemm, gemm, make_gemm
 
 __all__ = ["attn_bwd", "attn_fwd", "autotune_gemm", "gemm", "make_gemm"]
@@ -41,10 +42,12 @@ def attn_fwd(q, k, v, q_descale=None, k_descale=None, v_descale=None, causal=Fal
     Raises:
         NotImplementedError: If there is no kernel for the dtype or the GPU.
     """
-    from .attn import attn_fwd as _attn_fwd
-
+    args = (q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale)
+    done = fwd_api.common_case(*args, **config)
+    if done is not None:
+        return done
     _check(q, "forward", "attn_fwd")
-    return _attn_fwd(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config)
+    return fwd_api.attn_fwd(*args, **config)
 
 
 def attn_bwd(
@@ -59,9 +62,9 @@ def attn_bwd(
     Raises:
         NotImplementedError: If there is no kernel for the dtype or the GPU.
     """
-    from .attn import attn_bwd as _attn_bwd
-
+    args = (q, k, v, out, lse, pmax, dout, q_descale, k_descale, v_descale, causal, softmax_scale)
+    done = bwd_api.common_case(*args, **config)
+    if done is not None:
+        return done
     _check(q, "backward", "attn_bwd")
-    return _attn_bwd(
-        q, k, v, out, lse, pmax, dout, q_descale, k_descale, v_descale, causal, softmax_scale, **config
-    )
+    return bwd_api.attn_bwd(*args, **config)

@@ -131,6 +131,11 @@ def gemm_tune_key(kind, m, n, k, arch=100):
     return f"{kind}|m={m}|n={n}|k={k}|sm{arch}"
 
 
+def any_tuned():
+    """Whether the tune cache has any entry (so that a call without one need not build its key)."""
+    return bool(_entries())
+
+
 def tune_lookup(key):
     """The config stored under ``key``, or ``None``."""
     return _entries().get(key)
