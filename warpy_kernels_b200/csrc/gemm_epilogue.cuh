@@ -9,7 +9,9 @@
 // GELU is the exact erf form and its derivative cdf + x . pdf (warpy_kernels/utils/math.py:7-21).
 //
 // One thread owns one output row of the tile and walks it in chunks of 32 consecutive columns (the
-// layout tcgen05.ld 32x32b delivers), so a chunk is exactly one MX block.
+// layout tcgen05.ld 32x32b delivers), so a chunk is exactly one MX block.  A warp's chunk of a 16-bit output leaves
+// through 2 KiB of shared memory and a TMA store: stored straight from registers it is 32 rows of 64 bytes, whose
+// 128-byte lines cost the load/store unit 128 cycles a chunk and 4350 cycles a 128 x 256 tile.
 #pragma once
 #include <cuda_fp16.h>
 
@@ -57,39 +59,60 @@ __device__ __forceinline__ void unpack_half16x2(uint32_t w, float& lo, float& hi
   }
 }
 
-// Loads 32 consecutive 16-bit values of a row as fp32.
+// Loads 32 consecutive 16-bit values of a row (64-byte aligned) as fp32.
 template <bool F16>
 __device__ __forceinline__ void load_row32(const void* base, int64_t off, float (&x)[32]) {
-  const uint4* src = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(base) + off);
+  const uint16_t* src = static_cast<const uint16_t*>(base) + off;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const uint4 w = src[i];
+    const uint4 w = reinterpret_cast<const uint4*>(src)[i];
     unpack_half16x2<F16>(w.x, x[8 * i + 0], x[8 * i + 1]);
     unpack_half16x2<F16>(w.y, x[8 * i + 2], x[8 * i + 3]);
     unpack_half16x2<F16>(w.z, x[8 * i + 4], x[8 * i + 5]);
     unpack_half16x2<F16>(w.w, x[8 * i + 6], x[8 * i + 7]);
   }
 }
+
+constexpr int EPI_STAGE_BYTES = 32 * 64;  // one chunk of a warp: 32 rows x 32 16-bit values
+
+// Where a warp's chunks go.
+struct EpilogueTarget {
+  const CUtensorMap* out;  // 16-bit outputs in boxes of 32 columns x 32 rows, 64-byte swizzle
+  const CUtensorMap* pre;
+  uint32_t stage;          // the warp's EPI_STAGE_BYTES of shared memory, 512-byte aligned
+  int lane, row0;          // lane of the warp; the warp's first row
+};
+
+// Stores a chunk (every lane its row) as 16-bit values at column `col`.
 template <bool F16>
-__device__ __forceinline__ void store_row32(void* base, int64_t off, const float (&x)[32]) {
-  uint4* dst = reinterpret_cast<uint4*>(static_cast<uint16_t*>(base) + off);
+__device__ __forceinline__ void store_chunk(const EpilogueTarget& t, const CUtensorMap* map, int col,
+                                            const float (&x)[32]) {
+  if (t.lane == 0) bulk_wait_read_all();  // the previous chunk has left the buffer
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    uint4 w;
-    w.x = pack_half16x2<F16>(x[8 * i + 0], x[8 * i + 1]);
-    w.y = pack_half16x2<F16>(x[8 * i + 2], x[8 * i + 3]);
-    w.z = pack_half16x2<F16>(x[8 * i + 4], x[8 * i + 5]);
-    w.w = pack_half16x2<F16>(x[8 * i + 6], x[8 * i + 7]);
-    dst[i] = w;
+    // 16-byte pieces swizzled as the tensor map says (address bits 4-5 ^ bits 7-8), free of bank conflicts
+    const uint32_t dst = t.stage + t.lane * 64 + ((i ^ ((t.lane >> 1) & 3)) << 4);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst),
+                 "r"(pack_half16x2<F16>(x[8 * i + 0], x[8 * i + 1])), "r"(pack_half16x2<F16>(x[8 * i + 2], x[8 * i + 3])),
+                 "r"(pack_half16x2<F16>(x[8 * i + 4], x[8 * i + 5])), "r"(pack_half16x2<F16>(x[8 * i + 6], x[8 * i + 7]))
+                 : "memory");
+  }
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (t.lane == 0) {
+    tma_store_2d(map, t.stage, col, t.row0);
+    bulk_commit();
   }
 }
 
 // F16: fp16 instead of bf16 storage.  PLAIN: no column scales, no accumulation and no activation (the common
 // case, kept free of the tests for those options because the epilogue sits on the kernels' critical path).
 template <bool F16, bool PLAIN>
-__device__ __forceinline__ void epilogue_chunk_impl(const Epilogue& e, const uint32_t (&acc)[32], float row_scale,
-                                                    int row, int col, int N, void* out) {
-  const int64_t off = static_cast<int64_t>(row) * N + col;
+__device__ __forceinline__ void epilogue_chunk_impl(const Epilogue& e, const EpilogueTarget& t, const uint32_t (&acc)[32],
+                                                    float row_scale, int col, int N, const void* out) {
+  const int64_t row = t.row0 + t.lane;
+  const int64_t off = row * N + col;
   float f[32];
   if (!PLAIN && e.scale_b_cols) {
     const float4* sb = reinterpret_cast<const float4*>(e.scale_b + col);
@@ -112,7 +135,7 @@ __device__ __forceinline__ void epilogue_chunk_impl(const Epilogue& e, const uin
     for (int i = 0; i < 32; ++i) f[i] += c[i];
   }
   if (!PLAIN && e.act == ACT_GELU) {
-    if (e.pre_out) store_row32<F16>(e.pre_out, off, f);
+    if (e.pre_out) store_chunk<F16>(t, t.pre, col, f);
 #pragma unroll
     for (int i = 0; i < 32; ++i) f[i] = gelu_exact(f[i]);
   } else if (!PLAIN && e.act == ACT_DGELU) {
@@ -121,7 +144,7 @@ __device__ __forceinline__ void epilogue_chunk_impl(const Epilogue& e, const uin
 #pragma unroll
     for (int i = 0; i < 32; ++i) f[i] *= dgelu_exact(pre[i]);
   }
-  store_row32<F16>(out, off, f);
+  store_chunk<F16>(t, t.out, col, f);
   if (e.q_mx) {
     // this thread's 32 consecutive columns are exactly one MX block
     uint32_t amax = 0;
@@ -130,35 +153,29 @@ __device__ __forceinline__ void epilogue_chunk_impl(const Epilogue& e, const uin
     int ex = static_cast<int>((amax + 0x1fffffu) >> 23) - 8;
     ex = min(max(ex, 0), 254);
     const float inv = __uint_as_float(static_cast<uint32_t>(max(254 - ex, 1)) << 23);
-    uint4* qdst = reinterpret_cast<uint4*>(e.q_mx + off);
+    uint32_t w[8];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      uint4 w;
-      w.x = pack_e4m3x4(__fmul_rn(f[16 * i + 0], inv), __fmul_rn(f[16 * i + 1], inv), __fmul_rn(f[16 * i + 2], inv),
-                        __fmul_rn(f[16 * i + 3], inv));
-      w.y = pack_e4m3x4(__fmul_rn(f[16 * i + 4], inv), __fmul_rn(f[16 * i + 5], inv), __fmul_rn(f[16 * i + 6], inv),
-                        __fmul_rn(f[16 * i + 7], inv));
-      w.z = pack_e4m3x4(__fmul_rn(f[16 * i + 8], inv), __fmul_rn(f[16 * i + 9], inv),
-                        __fmul_rn(f[16 * i + 10], inv), __fmul_rn(f[16 * i + 11], inv));
-      w.w = pack_e4m3x4(__fmul_rn(f[16 * i + 12], inv), __fmul_rn(f[16 * i + 13], inv),
-                        __fmul_rn(f[16 * i + 14], inv), __fmul_rn(f[16 * i + 15], inv));
-      qdst[i] = w;
-    }
-    e.s_mx[static_cast<int64_t>(row) * (N / 32) + col / 32] = static_cast<uint8_t>(ex);
+    for (int i = 0; i < 8; ++i)
+      w[i] = pack_e4m3x4(__fmul_rn(f[4 * i + 0], inv), __fmul_rn(f[4 * i + 1], inv), __fmul_rn(f[4 * i + 2], inv),
+                         __fmul_rn(f[4 * i + 3], inv));
+    uint4* qdst = reinterpret_cast<uint4*>(e.q_mx + off);
+    qdst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    qdst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    e.s_mx[row * (N / 32) + col / 32] = static_cast<uint8_t>(ex);
   }
 }
 
-// acc: 32 fp32 accumulators (bit patterns) of row `row`, columns [col, col + 32).  `row_scale` = scalar scales and
-// the row's scale_a entry already multiplied together.  The branches are uniform over the grid.
-__device__ __forceinline__ void epilogue_chunk(const Epilogue& e, const uint32_t (&acc)[32], float row_scale, int row,
-                                               int col, int N, void* out) {
+// acc: 32 fp32 accumulators (bit patterns) of this lane's row, columns [col, col + 32).  `row_scale` = scalar scales
+// and the row's scale_a entry already multiplied together.  The branches are uniform over the grid.
+__device__ __forceinline__ void epilogue_chunk(const Epilogue& e, const EpilogueTarget& t, const uint32_t (&acc)[32],
+                                               float row_scale, int col, int N, const void* out) {
   const bool plain = !e.scale_b_cols && !e.accum && e.act == ACT_NONE;
   if (e.out_f16) {
-    epilogue_chunk_impl<true, false>(e, acc, row_scale, row, col, N, out);
+    epilogue_chunk_impl<true, false>(e, t, acc, row_scale, col, N, out);
   } else if (plain) {
-    epilogue_chunk_impl<false, true>(e, acc, row_scale, row, col, N, out);
+    epilogue_chunk_impl<false, true>(e, t, acc, row_scale, col, N, out);
   } else {
-    epilogue_chunk_impl<false, false>(e, acc, row_scale, row, col, N, out);
+    epilogue_chunk_impl<false, false>(e, t, acc, row_scale, col, N, out);
   }
 }
 

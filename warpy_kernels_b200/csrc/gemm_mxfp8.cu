@@ -1,245 +1,78 @@
-// MXFP8 block-scaled GEMM for sm_100a:
+// MXFP8 block-scaled GEMM for sm_100a: re-tiling of the scale factors and the C ABI entry points over the kernel in
+// gemm_core.cuh.
 //   out[M,N] = alpha . (a8 . 2^(sa-127)) . (b8 . 2^(sb-127))^T      bf16 output, fp32 accumulation
-// a8 [M,K], b8 [N,K] e4m3; sa [M,K/32], sb [N,K/32] ue8m0 bytes (one per row and 32
-// elements along K); either scale tensor may be absent (unit scales).  Optionally the
-// fp32 results are also written as MXFP8 (codes + scale byte per 32 columns) before
-// they are rounded to bf16.
+// a8 [M,K], b8 [N,K] e4m3; sa [M,K/32], sb [N,K/32] ue8m0 bytes (one per row and 32 elements along K); either scale
+// tensor may be absent (unit scales).  Optionally the fp32 results are also written as MXFP8 (codes + scale byte per
+// 32 columns) before they are rounded to bf16.
 //
-// Two kernels:
-//  1. swizzle_scales_kernel re-tiles the row-major scale bytes into the 512-byte
-//     atoms tcgen05.mma reads them in (128 rows x 4 K-blocks: byte offset
-//     (row % 32) * 16 + (row / 32 % 4) * 4 + kblock % 4), one atom per 128 rows and 128
-//     K elements, atoms ordered [row block][K block].  This is the kernel's scratch.
-//  2. gemm_mxfp8_kernel: persistent, warp-specialised, 128 x 256 tile, 128 K-bytes per
-//     stage.  Warp 0: TMA for A/B (128-byte swizzle) plus bulk copies of the scale
-//     atoms.  Warp 1: tcgen05.cp of the atoms into TMEM, then four
-//     tcgen05.mma kind::mxf8f6f4.block_scale (K = 32 each; the scale-factor id selects
-//     the byte of the K block).  Warps 2-5: epilogue from TMEM.
-//     TMEM: two 256-column accumulators that share 64 columns ([0,256) and [192,448)) plus the
-//     scale-factor columns.  The epilogue drains the shared columns of a tile first and then
-//     lets the next tile's main loop start while it drains the rest.
+// retile_scales_kernel turns the row-major scale bytes into the 512-byte atoms tcgen05.mma reads them in (128 rows x
+// 4 K-blocks: byte offset (row % 32) * 16 + (row / 32 % 4) * 4 + kblock % 4), one atom per 128 rows and 128 K elements,
+// atoms ordered [row block][K block].
 //
-// Arithmetic follows the reference's block-scaled path (warpy_kernels/gemm/sm120.py:121-146:
-// e4m3 products scaled by 2^(sfa-127) per row and 32-element K block, fp32 accumulate)
-// and its MX output epilogue (warpy_kernels/gemm/sm89.py:65-93).
+// Arithmetic follows the reference's block-scaled path (warpy_kernels/gemm/sm120.py:121-146: e4m3 products scaled by
+// 2^(sfa-127) per row and 32-element K block, fp32 accumulate) and its MX output epilogue
+// (warpy_kernels/gemm/sm89.py:65-93).
 //
 // Tensor-core bound: 2*M*N*K flops per launch.
-#include "common.cuh"
-#include "gemm_epilogue.cuh"
-#include "host_common.h"
-#include "gemm_mxfp8.h"
+#include "gemm_core.cuh"
 
 namespace wk {
 namespace {
 
-constexpr int BM = 128;
-constexpr int BN = 256;
-constexpr int BK = 128;  // bytes == e4m3 elements
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK;
-constexpr int B_BYTES = BN * BK;
-constexpr int SF_ATOM = 512;
-constexpr int SFA_BYTES = SF_ATOM;
-constexpr int SFB_BYTES = 2 * SF_ATOM;
-constexpr int STAGE_BYTES = A_BYTES + B_BYTES + SFA_BYTES + SFB_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 + 256;
-constexpr int THREADS = 192;
-constexpr int TMEM_COLS = 512;
-constexpr int ACC_STRIDE = 192;    // accumulator slot a lives in columns [192 a, 192 a + 256)
-constexpr int SF_COL = 448;        // scale-factor columns start here
-constexpr int SF_SLOTS = 4;        // one slot per smem stage
-constexpr int SF_SLOT_COLS = 12;   // 4 (A: 128 rows) + 8 (B: 256 rows)
+// ---------------------------------------------------------------------------
+// scale re-tiling
+// ---------------------------------------------------------------------------
+struct ScaleTensor {
+  const uint8_t* src;  // [rows, 4 num_kb] bytes, or null for unit scales
+  uint8_t* dst;        // atoms
+  int row_blocks;      // of 128 rows
+};
 
-// ---------------------------------------------------------------------------
-// scale pre-swizzle
-// ---------------------------------------------------------------------------
-// One thread per (row, 128-element K block): reads 4 scale bytes, writes one 32-bit word.
-__global__ void swizzle_scales_kernel(const uint8_t* __restrict__ s, uint32_t* __restrict__ out,
-                                      int rows, int kblocks128) {
-  const int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t total = static_cast<int64_t>(rows) * kblocks128;
-  if (idx >= total) return;
-  const int kb = static_cast<int>(idx % kblocks128);
-  const int row = static_cast<int>(idx / kblocks128);
-  uint32_t w = 0x7f7f7f7fu;  // unit scales when the caller gave none
-  if (s) w = *reinterpret_cast<const uint32_t*>(s + static_cast<int64_t>(row) * kblocks128 * 4 + kb * 4);
-  const int rb = row / 128;
-  const int r = row % 128;
-  const int64_t atom = static_cast<int64_t>(rb) * kblocks128 + kb;
-  out[atom * (SF_ATOM / 4) + (r % 32) * 4 + (r / 32)] = w;
+// One warp takes 128 rows x 4 K blocks: lane l reads the 16 scale bytes of rows l, l + 32, l + 64 and l + 96 and writes
+// their 16 bytes of each of four atoms, 2 KiB in a row per warp.  Both tensors of a product go in one launch.
+constexpr int RETILE_THREADS = 256;
+__global__ void __launch_bounds__(RETILE_THREADS)
+retile_scales_kernel(const ScaleTensor a, const ScaleTensor b, int num_kb) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x % 32;
+  const int groups = (num_kb + 3) / 4;
+  int64_t task = static_cast<int64_t>(blockIdx.x) * (RETILE_THREADS / 32) + threadIdx.x / 32;
+  const int64_t tasks_a = static_cast<int64_t>(a.row_blocks) * groups;
+  const bool second = task >= tasks_a;
+  if (second) task -= tasks_a;
+  const ScaleTensor& t = second ? b : a;
+  if (task >= static_cast<int64_t>(t.row_blocks) * groups) return;
+  const int rb = static_cast<int>(task / groups), kb = static_cast<int>(task % groups) * 4;
+  const int kbs = min(4, num_kb - kb);
+  uint32_t w[4][4];  // [row quarter][K block]
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint8_t* src = t.src + (static_cast<int64_t>(rb) * 128 + 32 * j + lane) * num_kb * 4 + kb * 4;
+    if (t.src && (num_kb & 3) == 0 && (reinterpret_cast<uintptr_t>(t.src) & 15) == 0) {
+      const uint4 v = *reinterpret_cast<const uint4*>(src);
+      w[j][0] = v.x, w[j][1] = v.y, w[j][2] = v.z, w[j][3] = v.w;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        w[j][i] = t.src && i < kbs ? *reinterpret_cast<const uint32_t*>(src + 4 * i) : 0x7f7f7f7fu;
+    }
+  }
+  uint4* dst = reinterpret_cast<uint4*>(t.dst + (static_cast<int64_t>(rb) * num_kb + kb) * SF_ATOM) + lane;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (i < kbs) dst[i * (SF_ATOM / 16)] = make_uint4(w[0][i], w[1][i], w[2][i], w[3][i]);
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                  const __grid_constant__ GemmParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + STAGES * STAGE_BYTES;
-  auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-  auto tfull_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + a); };
-  auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
-  const uint32_t ovl_bar = bar_base + 8u * (2 * STAGES + 4);  // the shared columns of the last tile are drained
-  const uint32_t tmem_slot = bar_base + 8u * (2 * STAGES + 5);
-
-  const int warp = threadIdx.x / 32;
-  const int lane = threadIdx.x % 32;
-  const int num_m = p.M / BM;
-  const int num_n = (p.N + BN - 1) / BN;
-  const int num_tiles = num_m * num_n;
-  const int num_kb = p.K / BK;
-  const int n_atoms_total = p.N / 128;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(tfull_bar(a), 1);
-      mbar_init(tempty_bar(a), 4);
-    }
-    mbar_init(ovl_bar, 4);
-    mbar_fence_init();
-    prefetch_tmap(&tmap_a);
-    prefetch_tmap(&tmap_b);
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  uint32_t tmem_base;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-
-  if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      // The launch may overlap the end of the kernel that re-tiles the scales (programmatic stream serialisation):
-      // nothing is loaded before that kernel has completed.
-      pdl_wait();
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
-        const TileCoord tc = tile_coord(tile, num_m, num_n, p.group_m);
-        const int nb_atoms = min(2, n_atoms_total - tc.n_blk * 2);  // 1 on a 128-wide edge tile
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(empty_bar(stage), phase ^ 1, p.status, WK_ERR_TIMEOUT_EMPTY)) {
-            ok = false;
-            break;
-          }
-          const uint32_t sa = smem_base + stage * STAGE_BYTES;
-          const uint32_t sb = sa + A_BYTES;
-          const uint32_t ssfa = sb + B_BYTES;
-          const uint32_t ssfb = ssfa + SFA_BYTES;
-          mbar_expect_tx(full_bar(stage), A_BYTES + B_BYTES + SFA_BYTES + nb_atoms * SF_ATOM);
-          tma_load_2d(sa, &tmap_a, full_bar(stage), kb * BK, tc.m_blk * BM);
-          tma_load_2d(sb, &tmap_b, full_bar(stage), kb * BK, tc.n_blk * BN);
-          bulk_load(ssfa, p.sfa + (static_cast<int64_t>(tc.m_blk) * num_kb + kb) * SF_ATOM, SF_ATOM,
-                    full_bar(stage));
-          for (int a = 0; a < nb_atoms; ++a) {
-            bulk_load(ssfb + a * SF_ATOM,
-                      p.sfb + (static_cast<int64_t>(tc.n_blk * 2 + a) * num_kb + kb) * SF_ATOM, SF_ATOM,
-                      full_bar(stage));
-          }
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
-        }
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      int local = 0;
-      bool ok = true;
-      // descriptors of stage 0; a later stage only moves the 16-byte-granular start address field
-      constexpr uint64_t kStageStep = STAGE_BYTES / 16;
-      static_assert(STAGE_BYTES % 16 == 0, "stage size must keep descriptors 16-byte granular");
-      const uint64_t a_desc0 = smem_desc_sw128(smem_base, 16, 1024);
-      const uint64_t b_desc0 = smem_desc_sw128(smem_base + A_BYTES, 16, 1024);
-      const uint64_t sfa_desc0 = smem_desc_plain(smem_base + A_BYTES + B_BYTES, 16, 128);
-      const uint64_t sfb_desc0 = smem_desc_plain(smem_base + A_BYTES + B_BYTES + SFA_BYTES, 16, 128);
-      for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++local) {
-        const int acc = local & 1;
-        // this slot was drained two tiles ago, and the previous tile has given up the columns it shares
-        if (!mbar_wait(tempty_bar(acc), ((local >> 1) & 1) ^ 1, p.status, WK_ERR_TIMEOUT_TMEM)) break;
-        if (local > 0 && !mbar_wait(ovl_bar, (local - 1) & 1, p.status, WK_ERR_TIMEOUT_TMEM)) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * ACC_STRIDE;
-        for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, p.status, WK_ERR_TIMEOUT_LOAD)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint64_t step = static_cast<uint64_t>(stage) * kStageStep;
-          const uint32_t sf_tmem = tmem_base + SF_COL + stage * SF_SLOT_COLS;
-          // 32 rows x 16 bytes per copy; the shared-memory source is a plain (unswizzled) block
-          tmem_cp_32x128b_warpx4(sf_tmem + 0, sfa_desc0 + step);
-          tmem_cp_32x128b_warpx4(sf_tmem + 4, sfb_desc0 + step);
-          tmem_cp_32x128b_warpx4(sf_tmem + 8, sfb_desc0 + step + SF_ATOM / 16);
-          const uint64_t a_desc = a_desc0 + step;
-          const uint64_t b_desc = b_desc0 + step;
-#pragma unroll
-          for (int k = 0; k < BK / 32; ++k) {
-            mma_mxf8_ss(d_tmem, a_desc + 2 * k, b_desc + 2 * k, make_idesc_mx(BM, BN, k, k), sf_tmem,
-                        sf_tmem + 4, (kb | k) != 0);
-          }
-          tc_commit(empty_bar(stage));
-          if (++stage == STAGES) {
-            stage = 0;
-            phase ^= 1;
-          }
-        }
-        if (ok) tc_commit(tfull_bar(acc));
-      }
-    }
-    __syncwarp();
-  } else {
-    const int quad = warp & 3;
-    int local = 0;
-    for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
-      const TileCoord tc = tile_coord(tile, num_m, num_n, p.group_m);
-      const int acc = local & 1;
-      if (!mbar_wait_warp(tfull_bar(acc), (local >> 1) & 1, p.status, WK_ERR_TIMEOUT_MMA)) break;
-      tc_fence_after();
-      // column chunks in the order they are drained: the 64 columns shared with the other slot first
-      const int first_chunk = acc == 0 ? 6 : 0;
-      const int row = tc.m_blk * BM + quad * 32 + lane;
-      const float row_scale = epilogue_row_scale(p.epi, row);
-#pragma unroll 1
-      for (int ci = 0; ci < BN / 32; ++ci) {
-        const int c = (ci + first_chunk) & 7;
-        uint32_t v[32];
-        tmem_ld32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * ACC_STRIDE + c * 32, v);
-        tc_wait_ld();
-        if (ci == 1) {
-          // both shared chunks are in registers: the next tile's main loop may overwrite them
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(ovl_bar);
-        }
-        const int col = tc.n_blk * BN + c * 32;
-        if (col < p.N) epilogue_chunk(p.epi, v, row_scale, row, col, p.N, p.out);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(tempty_bar(acc));
-    }
-  }
-
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
-  }
+int retile(const ScaleTensor& a, const ScaleTensor& b, int k, cudaStream_t st) {
+  int num_kb = k / 128;
+  const int64_t tasks = static_cast<int64_t>(a.row_blocks + b.row_blocks) * ((num_kb + 3) / 4);
+  if (tasks == 0) return 0;
+  const int64_t blocks = (tasks + RETILE_THREADS / 32 - 1) / (RETILE_THREADS / 32);
+  if (blocks > INT32_MAX) return WK_E_ARG;
+  return launch_pdl(reinterpret_cast<const void*>(retile_scales_kernel), dim3(static_cast<unsigned>(blocks)),
+                    RETILE_THREADS, 0, st, 1,
+                    {const_cast<ScaleTensor*>(&a), const_cast<ScaleTensor*>(&b), &num_kb});
 }
 
 Epilogue epilogue_of(const wk_gemm_mx_args* a) {
@@ -265,14 +98,15 @@ bool epilogue_args_ok(const wk_gemm_mx_args* a) {
   return true;
 }
 
-int swizzle(const void* s, void* dst, int rows, int k, cudaStream_t st) {
-  const int kb128 = k / 128;
-  const int64_t total = static_cast<int64_t>(rows) * kb128;
-  const int threads = 256;
-  const int64_t blocks = (total + threads - 1) / threads;
-  swizzle_scales_kernel<<<static_cast<unsigned>(blocks), threads, 0, st>>>(
-      static_cast<const uint8_t*>(s), static_cast<uint32_t*>(dst), rows, kb128);
-  return cudaGetLastError() == cudaSuccess ? 0 : WK_E_CUDA;
+GemmParams params_of(const wk_gemm_mx_args* a, int* status) {
+  GemmParams p = {};
+  p.out = a->out;
+  p.epi = epilogue_of(a);
+  p.M = a->m;
+  p.N = a->n;
+  p.group_m = a->group_m ? a->group_m : 8;
+  p.status = status;
+  return p;
 }
 
 }  // namespace
@@ -294,14 +128,15 @@ extern "C" int wk_tile_mx_scales(const void* s, int rows, int k, void* dst, void
   if (s && (reinterpret_cast<uintptr_t>(s) & 3)) return WK_E_ARG;
   if (rows == 0 || k == 0) return 0;
   if (int unsupported = require_sm100()) return unsupported;
-  return swizzle(s, dst, rows, k, static_cast<cudaStream_t>(stream));
+  const ScaleTensor t = {static_cast<const uint8_t*>(s), static_cast<uint8_t*>(dst), rows / 128}, none = {};
+  return retile(t, none, k, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int wk_gemm_mxfp8(const wk_gemm_mx_args* a, void* stream) {
   using namespace wk;
   if (!a) return WK_E_ARG;
   const int m = a->m, n = a->n, k = a->k;
-  if (m < 0 || n < 0 || k < 0 || m % BM || n % 128 || k % BK) return WK_E_ARG;
+  if (m < 0 || n < 0 || k < 0 || m % 128 || n % 128 || k % 128) return WK_E_ARG;
   if (m == 0 || n == 0) return 0;
   if (k == 0) return WK_E_ARG;
   if (!a->a || !a->b || !a->out) return WK_E_ARG;
@@ -315,7 +150,7 @@ extern "C" int wk_gemm_mxfp8(const wk_gemm_mx_args* a, void* stream) {
   if ((a->q_mx == nullptr) != (a->s_mx == nullptr)) return WK_E_ARG;
   if (a->q_mx && !aligned16(a->q_mx)) return WK_E_ARG;
   if (!epilogue_args_ok(a)) return WK_E_ARG;
-  if (a->cta_pair < 0 || a->cta_pair > 2) return WK_E_ARG;
+  if (a->cta_pair < 0 || a->cta_pair > 2 || a->group_m < 0) return WK_E_ARG;
   if (a->workspace && a->workspace_bytes < wk_gemm_mxfp8_workspace_bytes(m, n, k)) return WK_E_ARG;
   if (int unsupported = require_sm100()) return unsupported;
   int* status = status_word();
@@ -326,65 +161,19 @@ extern "C" int wk_gemm_mxfp8(const wk_gemm_mx_args* a, void* stream) {
   // re-tiled into the workspace first
   const uint8_t* sfa = static_cast<const uint8_t*>(a->a_scale_mx);
   const uint8_t* sfb = static_cast<const uint8_t*>(a->b_scale_mx);
-  int r = 0;
+  ScaleTensor ta = {}, tb = {};
   if (!a_tiled) {
-    uint8_t* dst = static_cast<uint8_t*>(a->workspace);
-    r = swizzle(a->a_scale_mx, dst, m, k, st);
-    if (r) return r;
-    sfa = dst;
+    ta = {sfa, static_cast<uint8_t*>(a->workspace), m / 128};
+    sfa = ta.dst;
   }
   if (!b_tiled) {
-    uint8_t* dst = static_cast<uint8_t*>(a->workspace) + ((static_cast<int64_t>(m) * (k / 32) + 15) / 16) * 16;
-    r = swizzle(a->b_scale_mx, dst, n, k, st);
-    if (r) return r;
-    sfb = dst;
+    tb = {sfb, static_cast<uint8_t*>(a->workspace) + ((static_cast<int64_t>(m) * (k / 32) + 15) / 16) * 16, n / 128};
+    sfb = tb.dst;
   }
+  if (int r = retile(ta, tb, k, st)) return r;
 
-  GemmParams p;
-  p.out = a->out;
-  p.sfa = sfa;
-  p.sfb = sfb;
-  p.epi = epilogue_of(a);
-  p.M = m;
-  p.N = n;
-  p.K = k;
-  if (a->group_m < 0) return WK_E_ARG;
-  p.group_m = a->group_m ? a->group_m : 8;
-  p.status = status;
-  if (a->cta_pair == 1) return launch_gemm_mxfp8_2sm(a->a, a->b, p, st, !(a_tiled && b_tiled));
-
-  CUtensorMap ta, tb;
-  {
-    const uint64_t dims[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(m)};
-    const uint64_t strides[1] = {static_cast<uint64_t>(k)};
-    const uint32_t box[2] = {BK, BM};
-    r = encode_tmap(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a->a, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (r) return r;
-  }
-  {
-    const uint64_t dims[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(n)};
-    const uint64_t strides[1] = {static_cast<uint64_t>(k)};
-    const uint32_t box[2] = {BK, BN};
-    r = encode_tmap(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a->b, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (r) return r;
-  }
-  if (allow_smem(reinterpret_cast<const void*>(gemm_mxfp8_kernel), SMEM_BYTES)) return WK_E_CUDA;
-  const int num_tiles = (m / BM) * ((n + BN - 1) / BN);
-  const int sms = sm_count();
-  if (sms <= 0) return WK_E_CUDA;
-  const int grid = num_tiles < sms ? num_tiles : sms;
-  // after a re-tiling launch: start under its tail (the producer waits for it before the first load)
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = (a_tiled && b_tiled) ? 0 : 1;
-  return cudaLaunchKernelEx(&cfg, gemm_mxfp8_kernel, ta, tb, p) == cudaSuccess ? 0 : WK_E_CUDA;
+  GemmParams p = params_of(a, status);
+  return launch_gemm<KIND_MX>(a->a, a->b, sfa, sfb, k, a->cta_pair, p, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -432,7 +221,7 @@ extern "C" int wk_gemm_mxfp8_noalloc(const wk_gemm_mx_args* a, void* stream) {
   using namespace wk;
   if (!a) return WK_E_ARG;
   const int m = a->m, n = a->n, k = a->k;
-  if (m < 0 || n < 0 || k < 0 || m % BM || n % 128 || k % BK) return WK_E_ARG;
+  if (m < 0 || n < 0 || k < 0 || m % 128 || n % 128 || k % 128) return WK_E_ARG;
   if (m == 0 || n == 0) return 0;
   if (k == 0) return WK_E_ARG;
   if (!a->a || !a->b || !a->out) return WK_E_ARG;
@@ -456,46 +245,12 @@ extern "C" int wk_gemm_mxfp8_noalloc(const wk_gemm_mx_args* a, void* stream) {
   uint8_t* sfa = g_noalloc_scratch_ptr[dev];
   uint8_t* sfb = sfa + ((static_cast<int64_t>(m) * (k / 32) + 15) / 16) * 16;
   // every atom the GEMM will read is rewritten here, so nothing of the previous call survives into this one
-  r = swizzle(a->a_scale_mx, sfa, m, k, st);
-  if (r) return r;
-  r = swizzle(a->b_scale_mx, sfb, n, k, st);
-  if (r) return r;
-
-  CUtensorMap ta, tb;
-  {
-    const uint64_t dims[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(m)};
-    const uint64_t strides[1] = {static_cast<uint64_t>(k)};
-    const uint32_t box[2] = {BK, BM};
-    r = encode_tmap(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a->a, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (r) return r;
-  }
-  {
-    const uint64_t dims[2] = {static_cast<uint64_t>(k), static_cast<uint64_t>(n)};
-    const uint64_t strides[1] = {static_cast<uint64_t>(k)};
-    const uint32_t box[2] = {BK, BN};
-    r = encode_tmap(&tb, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, a->b, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
-    if (r) return r;
-  }
-  GemmParams p;
-  p.out = a->out;
-  p.sfa = sfa;
-  p.sfb = sfb;
-  p.epi = epilogue_of(a);
-  p.M = m;
-  p.N = n;
-  p.K = k;
+  const ScaleTensor ta = {static_cast<const uint8_t*>(a->a_scale_mx), sfa, m / 128};
+  const ScaleTensor tb = {static_cast<const uint8_t*>(a->b_scale_mx), sfb, n / 128};
+  if ((r = retile(ta, tb, k, st))) return r;
+  GemmParams p = params_of(a, g_noalloc_status_ptr[dev]);
   p.group_m = 8;
-  p.status = g_noalloc_status_ptr[dev];
-  if (cudaFuncSetAttribute(reinterpret_cast<const void*>(gemm_mxfp8_kernel),
-                           cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess)
-    return WK_E_CUDA;
-  const int num_tiles = (m / BM) * ((n + BN - 1) / BN);
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-    return WK_E_CUDA;
-  const int grid = num_tiles < sms ? num_tiles : sms;
-  gemm_mxfp8_kernel<<<grid, THREADS, SMEM_BYTES, st>>>(ta, tb, p);
-  return cudaGetLastError() == cudaSuccess ? 0 : WK_E_CUDA;
+  return launch_gemm<KIND_MX>(a->a, a->b, sfa, sfb, k, 2, p, st);
 }
 
 extern "C" int wk_gemm_mxfp8_noalloc_status(void) {

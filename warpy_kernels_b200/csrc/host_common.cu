@@ -103,7 +103,7 @@ int sm_count() {
 
 int allow_smem(const void* func, int bytes) {
   // remembered per (kernel, device): the attribute belongs to the device's context
-  constexpr int kMaxFuncs = 32;
+  constexpr int kMaxFuncs = 64;
   static const void* funcs[kMaxFuncs] = {};
   static bool done[kMaxFuncs][kMaxDevices] = {};
   int dev = 0;
@@ -124,6 +124,59 @@ int allow_smem(const void* func, int bytes) {
     done[slot][dev] = true;
   }
   return 0;
+}
+
+int clusters_at_once(const void* func, int size, int threads, int smem) {
+  if (size == 1) return sm_count();  // every kernel that asks has one CTA per SM
+  constexpr int kMaxKnown = 64;
+  static struct {
+    const void* func;
+    int size, dev, n;
+  } known[kMaxKnown];
+  static int count = 0;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    for (int i = 0; i < count; ++i)
+      if (known[i].func == func && known[i].size == size && known[i].dev == dev) return known[i].n;
+  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = size;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(size);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, func, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::lock_guard<std::mutex> lock(g_mu);
+  if (count < kMaxKnown) known[count++] = {func, size, dev, n};
+  return n;
+}
+
+int launch_pdl(const void* func, dim3 grid, int threads, int smem, cudaStream_t stream, int cluster,
+               std::initializer_list<void*> args) {
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelExC(&cfg, func, const_cast<void**>(args.begin())) == cudaSuccess ? 0 : WK_E_CUDA;
 }
 
 }  // namespace wk

@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
+
 #include "../../include/warpy_b200.h"
 
 namespace wk {
@@ -28,8 +30,16 @@ int require_sm100();
 // Number of SMs of the current device (cached).
 int sm_count();
 
-// Raises the dynamic shared memory limit of `func` once per process.
+// Raises the dynamic shared memory limit of `func` once per device.
 int allow_smem(const void* func, int bytes);
+
+// How many clusters of `size` CTAs of this kernel the current device runs at once (asked once per device).
+int clusters_at_once(const void* func, int size, int threads, int smem);
+
+// Launches `func` in clusters of `cluster` CTAs as a programmatic dependent: it may be set up while the kernel before it
+// in the stream still runs, so it must execute griddepcontrol.wait before it touches global memory.
+int launch_pdl(const void* func, dim3 grid, int threads, int smem, cudaStream_t stream, int cluster,
+               std::initializer_list<void*> args);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
