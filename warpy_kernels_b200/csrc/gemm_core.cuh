@@ -553,9 +553,11 @@ struct GemmPlan {
 //
 // The model counts cycles: what a K block takes (the MMAs' time or the loads', whichever is longer), what a round of
 // tiles costs besides (first loads, epilogue) and what the exchange of partial sums adds.  Clusters of more than two
-// CTAs do not use all SMs: 45, 33, 22 and 15 clusters of 3, 4, 6 and 8 CTAs run at once on 148.
+// CTAs do not use all SMs: 45, 33, 22 and 15 clusters of 3, 4, 6 and 8 CTAs run at once on 148.  Over 39 shapes from
+// 128 x 640 x 2048 to 4096 x 2048 x 8192, bf16 and MXFP8, its choice is within 4 % of the best form but for one; a
+// single 128 x 256 CTA was never ahead of a pair or of narrow tiles by more than 1 %, so it runs on request only.
 inline GemmPlan gemm_plan(int m, int n, int num_kb, int sms, int force) {
-  GemmPlan best = {FORM_SINGLE, 1};
+  GemmPlan best = {FORM_PAIR, 1};
   double best_cycles = 1e30;
   auto consider = [&](int form, int s, double per_kb, double per_round, double once) {
     if (s > 1 && num_kb < 4 * s) return;  // a range of less than four K blocks is all start-up
@@ -572,11 +574,10 @@ inline GemmPlan gemm_plan(int m, int n, int num_kb, int sms, int force) {
       best = {form, s};
     }
   };
-  consider(FORM_SINGLE, 1, 580, 1500, 4000);
   consider(FORM_NARROW, 1, 400, 1500, 3500);
   consider(FORM_NARROW, 2, 400, 4500, 4500);
   consider(FORM_NARROW, 4, 400, 5000, 4500);
-  consider(FORM_PAIR, 1, 535, 1500, 6500);
+  consider(FORM_PAIR, 1, 535, 1500, 4500);
   consider(FORM_PAIR, 2, 535, 5500, 6500);
   consider(FORM_PAIR, 4, 535, 5500, 6500);
   if (force == 1) best.form = FORM_PAIR;
