@@ -1,0 +1,99 @@
+"""GPU: the attention forward for few query rows and small problems (packed query heads, keys split over warps and the
+CTAs of a cluster), FP8 and BF16: packed rows around multiples of 16, keys around multiples of a step, caches with
+lengths of their own down to 0, causal rows without a key, late peaks."""
+
+import pytest
+import torch
+
+from oracle import reference_math as R
+from tests.helpers import fwd_errors
+
+pytestmark = pytest.mark.gpu
+
+# (B, Hq, Hkv, Nq, Nk, d, causal)
+SHAPES = [
+    (1, 1, 1, 1, 1, 128, False), (1, 1, 1, 1, 33, 64, False), (3, 8, 1, 1, 500, 128, False),
+    (2, 16, 4, 1, 2049, 128, False), (1, 64, 8, 2, 4097, 128, True), (2, 4, 4, 3, 31, 64, True),
+    (1, 8, 2, 8, 1000, 128, True), (5, 2, 1, 16, 130, 64, False), (1, 4, 2, 33, 64, 128, True),
+    (1, 2, 1, 300, 777, 64, False), (1, 2, 1, 200, 90, 128, True), (40, 32, 8, 1, 700, 128, False),
+]
+
+
+def _inputs(cuda, shape, fp8, seed=0):
+    # not centred over the sequence as randn_qkv does it: with one key that leaves V = 0, and 0 / 0 for a cosine
+    B, Hq, Hkv, Nq, Nk, d = shape[:6]
+    g = torch.Generator(device=cuda).manual_seed(seed)
+    q, k, v = (torch.randn(B, h, n, d, device=cuda, generator=g) for h, n in ((Hq, Nq), (Hkv, Nk), (Hkv, Nk)))
+    if not fp8:
+        q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+        return (q, k, v), (q.float(), k.float(), v.float())
+    q8 = R.quantize_qkv(q, k, v)
+    return q8, R.dequantize_qkv(*q8)
+
+
+def _check(errs, fp8):
+    # P carries at least 11 (FP8) or 8 (BF16) bits here, so the output's own rounding to bf16 is what remains:
+    # the gates of the bf16 forward hold for both
+    assert errs["out"] <= 1e-2 and errs["lse"] <= 1e-2 and errs["max_abs"] <= 2e-2 and errs["cos"] >= 0.999, errs
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("shape", SHAPES)
+def test_matches_the_oracle(cuda, shape, fp8):
+    from warpy_kernels import attn_fwd
+
+    B, Hq, Hkv, Nq, Nk, d, causal = shape
+    args, deq = _inputs(cuda, shape, fp8)
+    out, lse, pmax = attn_fwd(*args, causal=causal)
+    out_ref, lse_ref = R.attention_reference(*deq, causal)
+    _check(fwd_errors(out, lse, out_ref, lse_ref, Nq, Nk, causal), fp8)
+    rep = Hq // Hkv
+    s = (deq[0] @ deq[1].repeat_interleave(rep, 1).transpose(-1, -2)) / d**0.5
+    if causal:
+        s = s.masked_fill(torch.arange(Nk, device=cuda) > torch.arange(Nq, device=cuda)[:, None] + Nk - Nq, float("-inf"))
+    seen = torch.isfinite(lse)
+    want = torch.softmax(s, -1).amax(-1)
+    assert torch.allclose(pmax[seen], want[seen], rtol=2e-3, atol=1e-6) and bool((pmax[~seen] == 0).all())
+    again = attn_fwd(*args, causal=causal)
+    assert all(torch.equal(x, y) for x, y in zip(again, (out, lse, pmax)))
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("causal", [False, True])
+def test_cache_lengths(cuda, fp8, causal):
+    """A [B, N, H, d] cache whose items attend to lengths of their own, the rest of it filled with large values."""
+    from warpy_kernels import attn_fwd
+
+    shape = (5, 16, 4, 2, 600, 128)
+    args, deq = _inputs(cuda, shape, fp8, seed=4)
+    used = [600, 1, 0, 257, 64]
+    k, v = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in args[1:3])
+    for b, n in enumerate(used):
+        k[b, :, n:] = torch.full_like(k[b, :, n:].float(), 400.0).to(k.dtype)
+        v[b, :, n:] = torch.full_like(v[b, :, n:].float(), -400.0).to(v.dtype)
+    lengths = torch.tensor(used, dtype=torch.int32, device=cuda)
+    out, lse, pmax = attn_fwd(args[0], k, v, *args[3:], causal=causal, seqused_k=lengths)
+    only = attn_fwd(args[0], k, v, *args[3:], causal=causal, seqused_k=lengths, return_lse=False)
+    assert torch.equal(only[0], out) and only[1] is None
+    for b, n in enumerate(used):
+        if n == 0:
+            assert bool((out[b] == 0).all()) and bool(torch.isinf(lse[b]).all()) and bool((pmax[b] == 0).all())
+            continue
+        out_ref, lse_ref = R.attention_reference(deq[0][b : b + 1], deq[1][b : b + 1, :, :n], deq[2][b : b + 1, :, :n], causal)
+        _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, 2, n, causal), fp8)
+
+
+@pytest.mark.parametrize("fp8", [True, False])
+def test_late_peaks(cuda, fp8):
+    """Scores hundreds of nats above the first ones: the reference moves, nothing is recomputed."""
+    from tests.test_attn_fwd_range_gpu import late_peak_qkv
+    from warpy_kernels import attn_fwd
+
+    q, k, v = late_peak_qkv(1, 8, 1, 1, 3000, 128, [(100, 90.0), (2000, 300.0)], device=cuda)
+    args = R.quantize_qkv(q, k, v) if fp8 else (q.bfloat16(), k.bfloat16(), v.bfloat16())
+    deq = R.dequantize_qkv(*args) if fp8 else tuple(x.float() for x in args)
+    out, lse, pmax = attn_fwd(*args)
+    out_ref, lse_ref = R.attention_reference(*deq, False)
+    errs = fwd_errors(out, lse, out_ref, lse_ref, 1, 3000, False)
+    assert errs["out"] <= 1e-2 and errs["lse"] <= 5e-2, errs  # lse near 400: fp32 logits in base 2
+    assert pmax.min().item() > 0.99

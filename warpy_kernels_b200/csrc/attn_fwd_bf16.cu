@@ -24,6 +24,7 @@
 #include <math.h>
 
 #include "attn_fwd_redo.h"
+#include "attn_rows.h"
 #include "common.cuh"
 #include "host_common.h"
 
@@ -432,6 +433,10 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
   }
   if (a->B > 65535 || a->Hq > 65535) return WK_E_ARG;
   if (int unsupported = require_sm100()) return unsupported;
+  if (a->workspace && (a->workspace_bytes < attn_fwd_flag_bytes(a->B, a->Hq, a->Nq) ||
+                       (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
+    return WK_E_ARG;
+  if (attn_rows_applies(a, true)) return launch_attn_rows(a, true, static_cast<cudaStream_t>(stream));
   int* status = status_word();
   if (!status) return WK_E_CUDA;
 
@@ -479,9 +484,6 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
   p.softmax_scale = a->softmax_scale;
   p.status = status;
   p.redo = static_cast<int*>(a->workspace);
-  if (a->workspace && (a->workspace_bytes < attn_fwd_flag_bytes(a->B, a->Hq, a->Nq) ||
-                       (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
-    return WK_E_ARG;
 
   const void* kernel = a->d == 64 ? reinterpret_cast<const void*>(attn_fwd_bf16_kernel<64>)
                                   : reinterpret_cast<const void*>(attn_fwd_bf16_kernel<128>);

@@ -45,6 +45,7 @@
 #include <type_traits>
 
 #include "attn_fwd_redo.h"
+#include "attn_rows.h"
 #include "common.cuh"
 #include "host_common.h"
 
@@ -1088,6 +1089,11 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   }
   if (a->B > 65535 || a->Hq > 65535) return WK_E_ARG;
   if (int unsupported = require_sm100()) return unsupported;
+  if (a->ctas_per_sm < 0 || a->ctas_per_sm > 2) return WK_E_ARG;
+  if (a->workspace && (a->workspace_bytes < attn_fwd_flag_bytes(a->B, a->Hq, a->Nq) ||
+                       (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
+    return WK_E_ARG;
+  if (attn_rows_applies(a, false)) return launch_attn_rows(a, false, static_cast<cudaStream_t>(stream));
   int* status = status_word();
   if (!status) return WK_E_CUDA;
 
@@ -1145,9 +1151,6 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   p.softmax_scale = a->softmax_scale;
   p.status = status;
   p.redo = static_cast<int*>(a->workspace);
-  if (a->workspace && (a->workspace_bytes < attn_fwd_flag_bytes(a->B, a->Hq, a->Nq) ||
-                       (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
-    return WK_E_ARG;
 
   const bool d64 = a->d == 64;
   const void* k_main = d64 ? reinterpret_cast<const void*>(attn_fwd_fp8_kernel<false, 64>)
@@ -1161,7 +1164,6 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   // against the two-CTA kernel: 1024 keys 723 / 1066 against 723 / 1070, 2048 keys 1012 / 1289 against 989 / 1253,
   // 4096 keys 1215 / 1412 against 1149 / 1342, 8192 keys 1321 / 1488 against 1192 / 1348, 16384 keys (causal) 1417
   // against 1140
-  if (a->ctas_per_sm < 0 || a->ctas_per_sm > 2) return WK_E_ARG;
   const bool wide = a->ctas_per_sm == 1 || (a->ctas_per_sm == 0 && a->Nk >= 2048);
   const int num_m = (a->Nq + BM - 1) / BM;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
