@@ -16,6 +16,9 @@ SHAPES = [
     (2, 16, 4, 1, 2049, 128, False), (1, 64, 8, 2, 4097, 128, True), (2, 4, 4, 3, 31, 64, True),
     (1, 8, 2, 8, 1000, 128, True), (5, 2, 1, 16, 130, 64, False), (1, 4, 2, 33, 64, 128, True),
     (1, 2, 1, 300, 777, 64, False), (1, 2, 1, 200, 90, 128, True), (40, 32, 8, 1, 700, 128, False),
+    # FP8 from 1024 keys on: products with the packed rows on the N side, 8 or 16 of them
+    (1, 1, 1, 1, 1024, 128, False), (2, 8, 1, 1, 1153, 64, False), (3, 9, 3, 3, 1500, 128, True),
+    (1, 32, 2, 2, 3333, 64, True), (20, 16, 2, 1, 1280, 128, False), (1, 2, 1, 8, 1031, 128, True),
 ]
 
 
@@ -60,17 +63,18 @@ def test_matches_the_oracle(cuda, shape, fp8):
 
 @pytest.mark.parametrize("fp8", [True, False])
 @pytest.mark.parametrize("causal", [False, True])
-def test_cache_lengths(cuda, fp8, causal):
-    """A [B, N, H, d] cache whose items attend to lengths of their own, the rest of it filled with large values."""
+@pytest.mark.parametrize("Nk,fill", [(600, 400.0), (1700, float("nan"))])
+def test_cache_lengths(cuda, fp8, causal, Nk, fill):
+    """A [B, N, H, d] cache whose items attend to lengths of their own, the rest of it filled with what must not count."""
     from warpy_kernels import attn_fwd
 
-    shape = (5, 16, 4, 2, 600, 128)
+    shape = (5, 16, 4, 2, Nk, 128)
     args, deq = _inputs(cuda, shape, fp8, seed=4)
-    used = [600, 1, 0, 257, 64]
+    used = [Nk, 1, 0, 257, 64]
     k, v = (x.transpose(1, 2).contiguous().transpose(1, 2) for x in args[1:3])
     for b, n in enumerate(used):
-        k[b, :, n:] = torch.full_like(k[b, :, n:].float(), 400.0).to(k.dtype)
-        v[b, :, n:] = torch.full_like(v[b, :, n:].float(), -400.0).to(v.dtype)
+        k[b, :, n:] = torch.full_like(k[b, :, n:].float(), fill).to(k.dtype)
+        v[b, :, n:] = torch.full_like(v[b, :, n:].float(), -fill).to(v.dtype)
     lengths = torch.tensor(used, dtype=torch.int32, device=cuda)
     out, lse, pmax = attn_fwd(args[0], k, v, *args[3:], causal=causal, seqused_k=lengths)
     only = attn_fwd(args[0], k, v, *args[3:], causal=causal, seqused_k=lengths, return_lse=False)

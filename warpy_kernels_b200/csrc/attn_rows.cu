@@ -422,6 +422,7 @@ attn_rows_kernel(const __grid_constant__ RowsParams p, int stages) {
 
 namespace {
 
+constexpr int R_DECODE_KEYS = 1024;  // from here on FP8 decoding goes to attn_decode.cu
 constexpr int R_DECODE_ROWS = 32;  // packed rows up to which the split is chosen to fill the GPU
 
 int rows_splits(const wk_attn_fwd_args* a, int sms) {
@@ -466,6 +467,8 @@ bool attn_rows_applies(const wk_attn_fwd_args* a, bool bf16) {
 }
 
 int launch_attn_rows(const wk_attn_fwd_args* a, bool bf16, cudaStream_t stream) {
+  if (!bf16 && a->Nk >= R_DECODE_KEYS && static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq <= R_DECODE_ROWS)
+    return launch_attn_decode(a, stream);
   const int sms = sm_count();
   if (sms <= 0) return WK_E_CUDA;
   RowsParams p = {};
