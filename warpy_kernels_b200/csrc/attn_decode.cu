@@ -13,7 +13,8 @@
 // softmax warp issues about 250 instructions.  The mma.sync form of the same split (attn_rows.cu), which converts K and
 // V to f16 in registers, issues 630 per 32 keys and warp and is bound by their latency.
 //
-// 192 threads, two CTAs per SM: warp 0 TMA producer (three stages of 128 keys), warp 1 MMA issue, warps 2-5 softmax.
+// 224 threads, two CTAs per SM: warp 0 TMA producer (three stages of 128 keys), warps 1 and 6 issue the two products,
+// warps 2-5 softmax.
 //
 // Numerics are those of attn_fwd_fp8.cu: P8 = e4m3(2^(s.beta - e_blk + 8)) with e_blk the exponent of the 32-key block,
 // O in units of the row reference m_ref, which is the row maximum of the split's first tile.  A split that meets a score
@@ -31,7 +32,7 @@ namespace {
 constexpr int E_KEYS = 128;  // keys per tile
 constexpr int E_STAGES = 3;
 constexpr int E_TILE_BYTES = E_KEYS * 128;  // rows of 128 bytes (head dimension 64: upper half zero, filled in by TMA)
-constexpr int E_THREADS = 192;
+constexpr int E_THREADS = 224;
 constexpr int E_SOFTMAX = 128;
 constexpr int E_P_OFFSET = 8;
 constexpr float E_MAX_EXP = 100.f;
@@ -206,43 +207,45 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       __syncwarp();
     } while (another_pass());
   } else if (warp == 1) {
+    // ---- S^T = K.Q^T, as soon as a tile and a buffer are there
     const bool mine = elect_one();
     constexpr uint32_t idesc_qk = make_idesc(0, 0, 0, 0, E_KEYS, C::QN);
     const uint64_t q_desc = smem_desc_sw128(q_smem, 16, 1024);
-    const uint32_t o_tmem = tmem_base + E_O_COL;
     bool ok = mbar_wait_warp(q_full, 0, p.status, WK_ERR_TIMEOUT_LOAD);
     do {
-      auto scores = [&](int j) -> bool {  // S^T of tile j into buffer j & 1
+      for (int j = base; ok && j < base + n_tiles; ++j) {
         const int s = j % E_STAGES, buf = j & 1;
-        if (!mbar_wait_warp(kv_full(s), (j / E_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) return false;
-        if (j >= 2 && !mbar_wait_warp(s_free(buf), ((j >> 1) - 1) & 1, p.status, WK_ERR_TIMEOUT_P)) return false;
+        if (j >= 2) ok = mbar_wait_warp(s_free(buf), ((j >> 1) - 1) & 1, p.status, WK_ERR_TIMEOUT_P);
+        ok = ok && mbar_wait_warp(kv_full(s), (j / E_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD);
         tc_fence_after();
-        if (mine) {
+        if (ok && mine) {
           const uint64_t k_desc = smem_desc_sw128(smem_base + s * 2 * E_TILE_BYTES, 16, 1024);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             if (32 * k < p.d) mma_f8_ss(tmem_base + E_S_COL + 32 * buf, k_desc + 2 * k, q_desc + 2 * k, idesc_qk, k != 0);
           tc_commit(s_full(buf));
         }
-        return true;
-      };
-      if (ok && n_tiles > 0) ok = scores(base);
+      }
+      __syncwarp();
+    } while (another_pass());
+  } else if (warp == 6) {
+    // ---- O^T += V^T.P^T.  By a warp of its own: one that also waits for the next tile's K before it gets here holds
+    // the stage back and with it the next load.
+    const bool mine = elect_one();
+    bool ok = true;
+    do {
       for (int j = base; ok && j < base + n_tiles; ++j) {
-        if (j + 1 < base + n_tiles) ok = scores(j + 1);
         const int s = j % E_STAGES, buf = j & 1;
-        if (!ok || !mbar_wait_warp(p_full(buf), (j >> 1) & 1, p.status, WK_ERR_TIMEOUT_P)) {
-          ok = false;
-          break;
-        }
+        ok = mbar_wait_warp(p_full(buf), (j >> 1) & 1, p.status, WK_ERR_TIMEOUT_P);
         tc_fence_after();
-        if (mine) {
+        if (ok && mine) {
           tmem_cp_32x128b_warpx4(tmem_base + E_SFB_COL + 4 * buf, smem_desc_plain(sf_smem + buf * C::SF_BYTES, 16, 128));
           // V tile: 128 keys (the MMA's K) x 128 bytes of head dimension (its M): MN-major, 32 keys = 4096 bytes
           const uint64_t v_desc = smem_desc_sw128(smem_base + s * 2 * E_TILE_BYTES + E_TILE_BYTES, 16, 1024);
           const uint64_t p_desc = smem_desc_sw128(p_smem + buf * C::P_BYTES, 16, 1024);
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            mma_mxf8_ss(o_tmem, v_desc + 256 * k, p_desc + 2 * k, make_idesc_mx_major(128, C::N, 0, k, 1, 0),
+            mma_mxf8_ss(tmem_base + E_O_COL, v_desc + 256 * k, p_desc + 2 * k, make_idesc_mx_major(128, C::N, 0, k, 1, 0),
                         tmem_base + E_SFA_COL, tmem_base + E_SFB_COL + 4 * buf, (j != base) | (k != 0));
           tc_commit(kv_empty(s));
           tc_commit(p_free(buf));
@@ -340,23 +343,30 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
         const uint32_t dst = p_smem + buf * C::P_BYTES + (r_key & 15);
         uint32_t my_sf = 0;  // lane r keeps the scale byte of row r
 #pragma unroll
-        for (int r = 0; r < NR; ++r) {
-          top[r] = fmaxf(top[r], cm[r]);
-          const bool live = cm[r] > -INFINITY;
-          float kf = live ? fminf(fmaxf(ceilf(cm[r] - m_ref[r]), -118.f), E_MAX_EXP) : 0.f;
-          const float bias = live ? static_cast<float>(E_P_OFFSET) - kf - m_ref[r] : 0.f;
-          const float x = ex2_approx(fmaf(__uint_as_float(raw[r]), beta, bias));
-          const int sf = live ? 127 + static_cast<int>(kf) - E_P_OFFSET : 0;
-          l[r] = fmaf(x, __uint_as_float(static_cast<uint32_t>(sf) << 23), l[r]);
-          const uint16_t hi = cvt_e4m3x2(x, 0.f);
-          float back, zero;
-          unpack_e4m3x2(hi, back, zero);
-          const uint16_t lo = cvt_e4m3x2((x - back) * 16.f, 0.f);
-          const uint32_t chunk = static_cast<uint32_t>(((r_key >> 4) ^ (r & 7)) << 4);
-          sts_u8(dst + r * 128 + chunk, hi);
-          sts_u8(dst + (NR + r) * 128 + chunk, lo);
-          if (lane == r) my_sf = static_cast<uint32_t>(sf);
-          if (lane == NR + r) my_sf = static_cast<uint32_t>(max(sf - 4, 0));
+        for (int r = 0; r < NR; r += 2) {  // two rows at a time: conversions work on pairs
+          float x[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            top[r + i] = fmaxf(top[r + i], cm[r + i]);
+            const bool live = cm[r + i] > -INFINITY;
+            const float kf = live ? fminf(fmaxf(ceilf(cm[r + i] - m_ref[r + i]), -118.f), E_MAX_EXP) : 0.f;
+            const float bias = live ? static_cast<float>(E_P_OFFSET) - kf - m_ref[r + i] : 0.f;
+            x[i] = ex2_approx(fmaf(__uint_as_float(raw[r + i]), beta, bias));
+            const int sf = live ? 127 + static_cast<int>(kf) - E_P_OFFSET : 0;
+            l[r + i] = fmaf(x[i], __uint_as_float(static_cast<uint32_t>(sf) << 23), l[r + i]);
+            if (lane == r + i) my_sf = static_cast<uint32_t>(sf);
+            if (lane == NR + r + i) my_sf = static_cast<uint32_t>(max(sf - 4, 0));
+          }
+          const uint16_t hi = cvt_e4m3x2(x[0], x[1]);
+          float b0, b1;
+          unpack_e4m3x2(hi, b0, b1);
+          const uint16_t lo = cvt_e4m3x2((x[0] - b0) * 16.f, (x[1] - b1) * 16.f);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const uint32_t at = dst + (r + i) * 128 + static_cast<uint32_t>(((r_key >> 4) ^ ((r + i) & 7)) << 4);
+            sts_u8(at, i ? hi >> 8 : hi);
+            sts_u8(at + NR * 128, i ? lo >> 8 : lo);
+          }
         }
         // scale bytes in the layout tcgen05.cp copies: row n at 16 n, key block at byte quad
         if (lane < C::N) sts_u8(sf_smem + buf * C::SF_BYTES + lane * 16 + quad, my_sf);

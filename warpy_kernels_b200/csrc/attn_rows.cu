@@ -35,6 +35,7 @@ constexpr int R_WARPS = 4;
 constexpr int R_THREADS = 32 * R_WARPS;
 constexpr int R_ROWS = 16;
 constexpr int R_RING_BYTES = 24 * 1024;  // per warp
+constexpr int R_MAX_SPLIT = 8;
 constexpr float R_P_SHIFT = 14.f;        // P is stored times 2^14 (FP8 inputs)
 
 struct RowsParams {
@@ -360,46 +361,68 @@ attn_rows_kernel(const __grid_constant__ RowsParams p, int stages) {
       part[R_ROWS * C::O_PITCH + 2 * R_ROWS + g + 8 * h] = top[h];
     }
   }
+  __syncthreads();
+  // Each CTA first merges its warps (local shared memory, a result behind theirs), then finishes the rows congruent to
+  // its rank from one partial result per CTA: all remote loads of a thread are independent of one another.
+  constexpr int QUADS = DH / 4;
+  float* merged = reinterpret_cast<float*>(smem_raw) + R_WARPS * C::PART_FLOATS;
+  constexpr int M_OFF = R_ROWS * C::O_PITCH, L_OFF = M_OFF + R_ROWS, T_OFF = L_OFF + R_ROWS;
+  for (int i = threadIdx.x; i < R_ROWS * QUADS; i += R_THREADS) {
+    const int r = i / QUADS, col = (i % QUADS) * 4;
+    const float* parts = reinterpret_cast<const float*>(smem_raw);
+    float mm = -INFINITY, m_true = -INFINITY, sum = 0.f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < R_WARPS; ++w) mm = fmaxf(mm, parts[w * C::PART_FLOATS + M_OFF + r]);
+#pragma unroll
+    for (int w = 0; w < R_WARPS; ++w) {
+      const float* x = parts + w * C::PART_FLOATS;
+      const float f = x[M_OFF + r] > -INFINITY ? exp2f(x[M_OFF + r] - mm) : 0.f;
+      const float4 c = *reinterpret_cast<const float4*>(x + r * C::O_PITCH + col);
+      acc.x = fmaf(c.x, f, acc.x), acc.y = fmaf(c.y, f, acc.y), acc.z = fmaf(c.z, f, acc.z), acc.w = fmaf(c.w, f, acc.w);
+      sum = fmaf(x[L_OFF + r], f, sum);
+      m_true = fmaxf(m_true, x[T_OFF + r]);
+    }
+    *reinterpret_cast<float4*>(merged + r * C::O_PITCH + col) = acc;
+    if (col == 0) merged[M_OFF + r] = mm, merged[L_OFF + r] = sum, merged[T_OFF + r] = m_true;
+  }
   if (p.splits > 1)
     cluster_sync();
   else
     __syncthreads();
-  // Each CTA finishes the rows congruent to its rank; a thread takes four columns, all partial results of the row in
-  // the order of split and warp.
-  constexpr int QUADS = DH / 4;
-  const int n_parts = p.splits * R_WARPS;
   for (int i = threadIdx.x; i < R_ROWS * QUADS; i += R_THREADS) {
     const int r = (i / QUADS) * p.splits + split, col = (i % QUADS) * 4;
     if (r >= R_ROWS || row0 + r >= rows) break;
-    auto from = [&](int part_index, int offset) -> uint32_t {
-      const uint32_t addr =
-          smem_u32(smem_raw) + static_cast<uint32_t>((part_index % R_WARPS) * C::PART_FLOATS + offset) * 4;
-      return p.splits > 1 ? mapa(addr, part_index / R_WARPS) : addr;
-    };
-    auto load = [&](uint32_t addr) {
-      float x;
-      asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(addr));
-      return x;
-    };
-    float mm = -INFINITY, m_true = -INFINITY, sum = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int x = 0; x < n_parts; ++x) {
-      mm = fmaxf(mm, load(from(x, R_ROWS * C::O_PITCH + r)));
-      m_true = fmaxf(m_true, load(from(x, R_ROWS * C::O_PITCH + 2 * R_ROWS + r)));
+    float mx[R_MAX_SPLIT], lx[R_MAX_SPLIT], tx[R_MAX_SPLIT], ox[R_MAX_SPLIT][4];
+#pragma unroll
+    for (int x = 0; x < R_MAX_SPLIT; ++x) {
+      mx[x] = tx[x] = -INFINITY;
+      lx[x] = ox[x][0] = ox[x][1] = ox[x][2] = ox[x][3] = 0.f;
+      if (x < p.splits) {
+        const uint32_t base = p.splits > 1 ? mapa(smem_u32(merged), x) : smem_u32(merged);
+        auto load = [&](int offset) {
+          float y;
+          asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(y) : "r"(base + offset * 4));
+          return y;
+        };
+        mx[x] = load(M_OFF + r), lx[x] = load(L_OFF + r), tx[x] = load(T_OFF + r);
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(ox[x][0]), "=f"(ox[x][1]), "=f"(ox[x][2]), "=f"(ox[x][3])
+                     : "r"(base + (r * C::O_PITCH + col) * 4));
+      }
     }
-#pragma unroll 4
-    for (int x = 0; x < n_parts; ++x) {
-      const float mx = load(from(x, R_ROWS * C::O_PITCH + r));
-      const float f = mx > -INFINITY ? exp2f(mx - mm) : 0.f;
-      sum = fmaf(load(from(x, R_ROWS * C::O_PITCH + R_ROWS + r)), f, sum);
-      float c0, c1, c2, c3;
-      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                   : "=f"(c0), "=f"(c1), "=f"(c2), "=f"(c3)
-                   : "r"(from(x, r * C::O_PITCH + col)));
-      acc[0] = fmaf(c0, f, acc[0]);
-      acc[1] = fmaf(c1, f, acc[1]);
-      acc[2] = fmaf(c2, f, acc[2]);
-      acc[3] = fmaf(c3, f, acc[3]);
+    float mm = -INFINITY, m_true = -INFINITY, sum = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int x = 0; x < R_MAX_SPLIT; ++x) {
+      mm = fmaxf(mm, mx[x]);
+      m_true = fmaxf(m_true, tx[x]);
+    }
+#pragma unroll
+    for (int x = 0; x < R_MAX_SPLIT; ++x) {
+      const float f = mx[x] > -INFINITY ? exp2f(mx[x] - mm) : 0.f;
+      sum = fmaf(lx[x], f, sum);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[c] = fmaf(ox[x][c], f, acc[c]);
     }
     const bool empty = !(sum > 0.f);
     const float inv = empty ? 0.f : (FP8 ? p.v_descale[sc] : 1.f) / sum;
@@ -428,10 +451,15 @@ constexpr int R_DECODE_ROWS = 32;  // packed rows up to which the split is chose
 int rows_splits(const wk_attn_fwd_args* a, int sms) {
   const int64_t rows = static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq;
   const int64_t units = static_cast<int64_t>(a->B) * a->Hkv * ((rows + R_ROWS - 1) / R_ROWS);
-  if (rows > R_DECODE_ROWS) return 4;
+  if (rows > R_DECODE_ROWS) {
+    // A small problem: from the rows alone, so that a batch item attends to its seqused_k keys in the same order as a
+    // call on the truncated tensors does.
+    const int64_t per_item = static_cast<int64_t>(a->Hkv) * ((rows + R_ROWS - 1) / R_ROWS);
+    return per_item <= 40 ? 4 : per_item <= sms ? 2 : 1;
+  }
   // two CTAs of four warps per SM; at least 128 keys for a CTA
   int s = 1;
-  while (s < 8 && units * s * 2 <= 2 * sms && a->Nk >= 256 * s) s *= 2;
+  while (s < R_MAX_SPLIT && units * s * 2 <= 2 * sms && a->Nk >= 256 * s) s *= 2;
   return s;
 }
 
@@ -444,7 +472,7 @@ int launch_rows(RowsParams& p, cudaStream_t stream) {
   const int per_warp = (steps + R_WARPS * p.splits - 1) / (R_WARPS * p.splits);
   int stages = per_warp < 3 ? per_warp : per_warp < 6 ? 3 : C::MAX_STAGES;
   if (stages > C::MAX_STAGES) stages = C::MAX_STAGES;
-  const int ring = R_WARPS * stages * C::STAGE_BYTES, parts = R_WARPS * C::PART_FLOATS * 4;
+  const int ring = R_WARPS * stages * C::STAGE_BYTES, parts = (R_WARPS + 1) * C::PART_FLOATS * 4;
   const int smem = ring > parts ? ring : parts;
   const int most = R_WARPS * R_RING_BYTES > parts ? R_WARPS * R_RING_BYTES : parts;
   if (allow_smem(fn, most)) return WK_E_CUDA;
@@ -463,7 +491,9 @@ bool attn_rows_applies(const wk_attn_fwd_args* a, bool bf16) {
   const int64_t kv = static_cast<int64_t>(a->B) * a->Hkv;
   if (kv > 65535 || rows > 16 * 65535) return false;
   if (rows <= R_DECODE_ROWS) return true;
-  return kv * rows * a->Nk <= (1 << 20);
+  // Against the tensor-core kernels with their 128-row tiles (us, FP8): d 64, 600 x 777: 9 / 15, 2048 x 2048 causal
+  // 13 / 22; d 128, 128 x 128 7 / 15, but 1024 x 512 x 2 23 / 15 and 1536 x 640 x 2 20 / 19.
+  return kv * rows * a->Nk <= (a->d == 64 ? 1 << 22 : 1 << 20);
 }
 
 int launch_attn_rows(const wk_attn_fwd_args* a, bool bf16, cudaStream_t stream) {
