@@ -17,13 +17,13 @@
 // reference moves its reference exponent with the running maximum and rescales O, this kernel fixes m_ref per
 // row at the maximum of the first tile and never rescales: bf16 has the exponent range of fp32, so
 // P = 2^(s.beta - m_ref) keeps its eight significant bits whether it lies above or below 1.  Scores that outgrow
-// m_ref by more than 2^100 make the kernel flag the query block in the call's workspace, and attn_fwd_redo.cu
-// computes it again with the exact row maximum (without a workspace: WK_ERR_RANGE in the status word).
+// m_ref by more than 2^100 make the kernel compute the row again with the exact row maximum (attn_fwd_exact.cuh; for a
+// caller without a workspace: WK_ERR_RANGE in the status word).
 //
 // Tensor-core bound: 4 . B . Hq . Nq . Nk . d flops (half of that when causal).
 #include <math.h>
 
-#include "attn_fwd_redo.h"
+#include "attn_fwd_exact.cuh"
 #include "attn_rows.h"
 #include "common.cuh"
 #include "host_common.h"
@@ -66,7 +66,7 @@ struct FwdParams {
   float softmax_scale;
   int m_first;  // first query block of this launch (the grid covers gridDim.x blocks from here)
   int* status;
-  int* redo;    // one flag per query block, or null: blocks whose scores outgrow the row reference are recomputed
+  ExactInputs exact;  // rows whose scores outgrow the row reference
 };
 
 // One block of 32 keys of one row: P as 16 bf16 pairs and the sum of the unrounded values.
@@ -137,6 +137,7 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
+  pdl_wait();
   const int m_blk = p.m_first + gridDim.x - 1 - blockIdx.x;  // longest (latest) causal blocks first
   const int hq = blockIdx.y;
   const int b = blockIdx.z;
@@ -356,17 +357,13 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       l += l_o;
       m_true = fmaxf(m_true, mt_o);
     }
-    if (grp == 0 && m_true - m_ref > MAX_BLOCK_EXP) {
-      // Some key lies more than 2^100 above the first tile's maximum: P has overflowed bf16.  With a flag array the
-      // block is computed again (attn_fwd_redo.cu) and what is stored below is overwritten.
-      if (p.redo)
-        p.redo[attn_fwd_flag_index(b, hq, m_blk, p.Hq, (p.Nq + BM - 1) / BM)] = 1;
-      else
-        atomicCAS(p.status, 0, WK_ERR_RANGE);
-    }
+    // Some key lies more than 2^100 above the first tile's maximum: P has overflowed bf16.
+    const bool far = m_true - m_ref > MAX_BLOCK_EXP;
+    if (far && !p.exact.flags) atomicCAS(p.status, 0, WK_ERR_RANGE);
+    const bool exact = far && p.exact.flags;
     if (ok) {
       tc_fence_after();
-      const bool empty = !(l > 0.f);
+      const bool empty = !exact && !(l > 0.f);
       const float inv = empty ? 0.f : 1.f / l;
       const int col0 = (DH / 2) * grp;
       __nv_bfloat16* out_row = p.out + b * p.out_stride_b + hq * p.out_stride_h +
@@ -381,7 +378,12 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
-        if (row < p.Nq) {
+        if (row < p.Nq && exact) {
+          const ExactRow x = exact_row32<true>(p.exact, b, hq, hkv, row, min(row_limit, nk - 1), beta, 1.f, col0 + c * 32,
+                                               out_row + c * 32);
+          m_ref = m_true = x.m;
+          l = x.l;
+        } else if (row < p.Nq) {
           uint4* dst = reinterpret_cast<uint4*>(out_row + c * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -433,7 +435,7 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
   }
   if (a->B > 65535 || a->Hq > 65535) return WK_E_ARG;
   if (int unsupported = require_sm100()) return unsupported;
-  if (a->workspace && (a->workspace_bytes < attn_fwd_flag_bytes(a->B, a->Hq, a->Nq) ||
+  if (a->workspace && (a->workspace_bytes < wk_attn_fwd_workspace_bytes(a->B, a->Hq, a->Nq) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
     return WK_E_ARG;
   if (attn_rows_applies(a, true)) return launch_attn_rows(a, true, static_cast<cudaStream_t>(stream));
@@ -483,17 +485,13 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
   p.seqused_k = a->seqused_k;
   p.softmax_scale = a->softmax_scale;
   p.status = status;
-  p.redo = static_cast<int*>(a->workspace);
+  p.exact = exact_inputs(a, 2);
 
   const void* kernel = a->d == 64 ? reinterpret_cast<const void*>(attn_fwd_bf16_kernel<64>)
                                   : reinterpret_cast<const void*>(attn_fwd_bf16_kernel<128>);
   if (allow_smem(kernel, SMEM_BYTES)) return WK_E_CUDA;
   const int num_m = (a->Nq + BM - 1) / BM;
   p.m_first = 0;
-  dim3 grid(num_m, a->Hq, a->B);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  void* args[] = {&tq, &tk, &tv, &p};
-  if (cudaLaunchKernel(kernel, grid, dim3(THREADS), args, SMEM_BYTES, st) != cudaSuccess) return WK_E_CUDA;
-  // blocks the kernel flagged as beyond its exponent range are computed again (normally none)
-  return p.redo ? launch_attn_fwd_redo(a, true, p.redo, st) : 0;
+  return launch_pdl(kernel, dim3(num_m, a->Hq, a->B), THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream), 1,
+                    {&tq, &tk, &tv, &p});
 }

@@ -33,9 +33,8 @@
 // reference m_ref per row.  m_ref is the row maximum of the first tile (its largest
 // probability is then stored exactly, 2^8, as in the reference) and never moves: block
 // exponents above it are as good as below it.  Scores that outgrow it by more than 2^100
-// (69 nats) cannot be represented; the kernel then flags the query block in the call's workspace and the block is
-// computed again by attn_fwd_redo.cu with the exact row maximum (without a workspace: WK_ERR_RANGE in the status
-// word).  Query blocks that see at most 512 keys carry P as two
+// (69 nats) cannot be represented; such a row is computed again with its exact maximum (attn_fwd_exact.cuh; for a caller
+// without a workspace: WK_ERR_RANGE in the status word).  Query blocks that see at most 512 keys carry P as two
 // e4m3 terms (value + 2^-4 . residual): with so few keys the rounding of P would not
 // average out.
 //
@@ -44,7 +43,7 @@
 
 #include <type_traits>
 
-#include "attn_fwd_redo.h"
+#include "attn_fwd_exact.cuh"
 #include "attn_rows.h"
 #include "common.cuh"
 #include "host_common.h"
@@ -122,18 +121,9 @@ struct FwdParams {
   float softmax_scale;
   int m_first;  // first query block of this launch (the grid covers gridDim.x blocks from here)
   int* status;
-  int* redo;    // one flag per query block, or null: blocks whose scores outgrow the row reference are recomputed
+  int first_in_call;  // no kernel of this call before this one: wait for the stream's earlier work
+  ExactInputs exact;  // rows whose scores outgrow the row reference
 };
-
-// Some key of the row lies more than 2^MAX_BLOCK_EXP above the row reference: with a flag array the query block is
-// marked for recomputation (attn_fwd_redo.cu) and what this kernel stores for it is overwritten; without one the
-// status word says that the result is not to be trusted.
-__device__ __noinline__ void report_out_of_range(const FwdParams& p, int b, int hq, int m_blk) {
-  if (p.redo)
-    p.redo[attn_fwd_flag_index(b, hq, m_blk, p.Hq, (p.Nq + 127) / 128)] = 1;
-  else
-    atomicCAS(p.status, 0, WK_ERR_RANGE);
-}
 
 // One block of 32 keys of one row: P codes (and the residual codes) and the sum of the exact values.
 template <bool RESID>
@@ -214,6 +204,7 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
+  if (p.first_in_call) pdl_wait();
   const int m_blk = p.m_first + gridDim.x - 1 - blockIdx.x;  // longest (latest) causal blocks first
   const int hq = blockIdx.y;
   const int b = blockIdx.z;
@@ -455,10 +446,12 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       l += l_o;
       m_true = fmaxf(m_true, mt_o);
     }
-    if (grp == 0 && m_true - m_ref > MAX_BLOCK_EXP) report_out_of_range(p, b, hq, m_blk);
+    const bool far = m_true - m_ref > MAX_BLOCK_EXP;  // some key of the row is out of range (attn_fwd_exact.cuh)
+    if (far && !p.exact.flags) atomicCAS(p.status, 0, WK_ERR_RANGE);
+    const bool exact = far && p.exact.flags;
     if (ok) {
       tc_fence_after();
-      const bool empty = !(l > 0.f);
+      const bool empty = !exact && !(l > 0.f);
       const float inv = empty ? 0.f : sv / l;
       const int col0 = (DH / 2) * grp;
       __nv_bfloat16* out_row = p.out + b * p.out_stride_b + hq * p.out_stride_h +
@@ -473,7 +466,12 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
-        if (row < p.Nq) {
+        if (row < p.Nq && exact) {
+          const ExactRow x = exact_row32<false>(p.exact, b, hq, hkv, row, min(row_limit, nk - 1), beta, sv, col0 + c * 32,
+                                               out_row + c * 32);
+          m_ref = m_true = x.m;
+          l = x.l;
+        } else if (row < p.Nq) {
           uint4* dst = reinterpret_cast<uint4*>(out_row + c * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -550,6 +548,7 @@ struct WideItem {
 };
 
 constexpr int M_SCHED_SLOTS = 4;  // answers of the launch control in flight
+constexpr int M_MARK_OFFSET = 8 * (1 + 2 * M_SCHED_SLOTS) + 4;  // "a block is marked", from the sum_meet barrier on
 constexpr int M_CONSUMERS = 3 + M_SOFTMAX_THREADS;  // threads that read every answer
 
 // The query block of grid index (x, y, z); false if it belongs to the two-term variant's launch.
@@ -570,6 +569,45 @@ __device__ __forceinline__ bool wide_item(const FwdParams& p, uint32_t x, uint32
   it.n_tiles = n_tiles;
   it.n_rounds = (n_tiles + 1) / 2;  // 128 keys each; the second half of the last one may be all masked
   return n_tiles > RESID_MAX_TILES;
+}
+
+// Some key of a row lies more than 2^MAX_BLOCK_EXP above the row reference: the query block is marked in the workspace as
+// this CTA's, and the CTA recomputes it at its end (attn_fwd_exact.cuh).
+__device__ __noinline__ void wide_mark_block(const FwdParams& p, int b, int hq, int m_blk, uint32_t sum_meet) {
+  if (p.exact.flags) {
+    const int cta = 1 + blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    p.exact.flags[(b * p.Hq + hq) * ((p.Nq + BM - 1) / BM) + m_blk] = cta;
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(sum_meet + M_MARK_OFFSET), "r"(1) : "memory");
+  } else {
+    atomicCAS(p.status, 0, WK_ERR_RANGE);
+  }
+}
+
+// Recomputes the query blocks this CTA has marked, every softmax thread 32 columns of a row, and takes the marks back.
+__device__ __noinline__ void wide_recompute(const FwdParams& p, int row_in_block, int grp) {
+  const int num_m = (p.Nq + BM - 1) / BM;
+  const int cta = 1 + blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  for (int i = 0; i < p.B * p.Hq * num_m; ++i) {
+    if (p.exact.flags[i] != cta) continue;
+    const int row = (i % num_m) * BM + row_in_block, hq = (i / num_m) % p.Hq, b = i / (num_m * p.Hq);
+    const int hkv = hq / (p.Hq / p.Hkv), sc = b * p.Hkv + hkv, col0 = 32 * grp;
+    const int nk = p.seqused_k ? max(0, min(p.Nk, p.seqused_k[b])) : p.Nk;
+    if (row < p.Nq && col0 < p.d) {
+      const float beta = p.softmax_scale * p.q_descale[sc] * p.k_descale[sc] * 1.4426950408889634f;
+      const ExactRow x = exact_row32<false>(
+          p.exact, b, hq, hkv, row, p.causal ? min(row + nk - p.Nq, nk - 1) : nk - 1, beta, p.v_descale[sc], col0,
+          p.out + b * p.out_stride_b + hq * p.out_stride_h + static_cast<int64_t>(row) * p.out_stride_n + col0);
+      if (p.write_lse && grp == 0) {
+        const int64_t off = b * p.lse_stride_b + hq * p.lse_stride_h + row;
+        const bool empty = !(x.l > 0.f);
+        const float lse = empty ? INFINITY : x.m + log2f(x.l);
+        p.lse[off] = p.lse_natural ? lse * 0.6931471805599453f : lse;
+        p.pmax[off] = empty ? 0.f : exp2f(x.m - lse);
+      }
+    }
+    asm volatile("bar.sync 1, 512;" ::: "memory");  // every softmax thread has seen the mark
+    if (row_in_block == 0 && grp == 0) p.exact.flags[i] = 0;
+  }
 }
 
 // Stores a finished query block's output (called by every softmax thread: group `grp` stores head-dim columns
@@ -596,7 +634,7 @@ __device__ __noinline__ bool wide_store_output(const FwdParams& p, uint32_t xch,
     l += l_g;
     m_true = fmaxf(m_true, mt_g);
   }
-  if (grp == 0 && m_true - m_ref > MAX_BLOCK_EXP) report_out_of_range(p, b, hq, row / BM);
+  if (grp == 0 && m_true - m_ref > MAX_BLOCK_EXP) wide_mark_block(p, b, hq, row / BM, sum_meet);
   if (!mbar_wait_warp(o_full, fin_ci & 1, p.status, WK_ERR_TIMEOUT_MMA)) return false;
   tc_fence_after();
   const bool empty = !(l > 0.f);
@@ -694,6 +732,7 @@ attn_fwd_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     mbar_init(o_free, M_SOFTMAX_THREADS);
     mbar_init(ref_full, GROUP_THREADS);
     mbar_init(sum_meet, M_SOFTMAX_THREADS);
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(sum_meet + M_MARK_OFFSET), "r"(0) : "memory");
     mbar_fence_init();
     prefetch_tmap(&tmap_q);
     prefetch_tmap(&tmap_k);
@@ -708,6 +747,7 @@ attn_fwd_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  if (p.first_in_call) pdl_wait();
 
   WideItem it;
   bool ok = true;
@@ -1053,6 +1093,11 @@ attn_fwd_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     tc_fence_after();
     tmem_dealloc(tmem_base, M_TMEM_COLS);
   }
+  if (warp >= 3) {
+    uint32_t marked;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(marked) : "r"(sum_meet + M_MARK_OFFSET) : "memory");
+    if (marked) wide_recompute(p, (warp & 3) * 32 + lane, (warp - 3) >> 2);
+  }
   pdl_wait();  // does not end before the two-term launch, which started before this one, has
 }
 
@@ -1090,7 +1135,7 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   if (a->B > 65535 || a->Hq > 65535) return WK_E_ARG;
   if (int unsupported = require_sm100()) return unsupported;
   if (a->ctas_per_sm < 0 || a->ctas_per_sm > 2) return WK_E_ARG;
-  if (a->workspace && (a->workspace_bytes < attn_fwd_flag_bytes(a->B, a->Hq, a->Nq) ||
+  if (a->workspace && (a->workspace_bytes < wk_attn_fwd_workspace_bytes(a->B, a->Hq, a->Nq) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
     return WK_E_ARG;
   if (attn_rows_applies(a, false)) return launch_attn_rows(a, false, static_cast<cudaStream_t>(stream));
@@ -1150,7 +1195,7 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   p.seqused_k = a->seqused_k;
   p.softmax_scale = a->softmax_scale;
   p.status = status;
-  p.redo = static_cast<int*>(a->workspace);
+  p.exact = exact_inputs(a, 1);
 
   const bool d64 = a->d == 64;
   const void* k_main = d64 ? reinterpret_cast<const void*>(attn_fwd_fp8_kernel<false, 64>)
@@ -1160,12 +1205,16 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   const void* k_wide = reinterpret_cast<const void*>(attn_fwd_fp8_wide_kernel);
   if (allow_smem(k_main, SMEM_BYTES) || allow_smem(k_resid, SMEM_BYTES) || allow_smem(k_wide, M_SMEM_BYTES))
     return WK_E_CUDA;
-  // ctas_per_sm: 0 picks by the number of keys.  Measured with equal work (causal / full, TFLOP/s), the wide kernel
-  // against the two-CTA kernel: 1024 keys 723 / 1066 against 723 / 1070, 2048 keys 1012 / 1289 against 989 / 1253,
-  // 4096 keys 1215 / 1412 against 1149 / 1342, 8192 keys 1321 / 1488 against 1192 / 1348, 16384 keys (causal) 1417
-  // against 1140
-  const bool wide = a->ctas_per_sm == 1 || (a->ctas_per_sm == 0 && a->Nk >= 2048);
+  // ctas_per_sm: 0 picks.  Measured with equal work on a full GPU (causal / full, TFLOP/s), the wide kernel against the
+  // two-CTA kernel: 1024 keys 723 / 1066 against 723 / 1070, 2048 keys 1012 / 1289 against 989 / 1253, 4096 keys
+  // 1215 / 1412 against 1149 / 1342, 8192 keys 1321 / 1488 against 1192 / 1348, 16384 keys (causal) 1417 against 1140.
+  // A problem with no more query blocks than SMs has one CTA per SM either way, and then the wide kernel's four softmax
+  // groups are ahead from the start (1000 x 1000 x 4 heads 15.5 / 16.5 us against 18.5 / 22.5).
   const int num_m = (a->Nq + BM - 1) / BM;
+  const int sms = sm_count();
+  if (sms <= 0) return WK_E_CUDA;
+  const bool few = static_cast<int64_t>(num_m) * a->Hq * a->B <= sms;
+  const bool wide = a->ctas_per_sm == 1 || (a->ctas_per_sm == 0 && (a->Nk >= 2048 || few));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Query blocks that see few key tiles run the two-term variant.  The tile count never decreases with the
   // block index, so without per-batch key lengths the two variants get disjoint block ranges; with seqused_k
@@ -1187,31 +1236,22 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   const int resid_count = a->seqused_k ? num_m : m_split;
   // The short blocks first: their CTAs are many and brief, and the main launch, allowed to start while they still
   // run (programmatic stream serialisation), fills the SMs as they leave instead of waiting for the last of them.
+  p.first_in_call = 1;
   if (resid_count > 0) {
     p.m_first = 0;
-    void* args[] = {&tq, &tk, &tv, &p};
-    if (cudaLaunchKernel(k_resid, dim3(resid_count, a->Hq, a->B), dim3(THREADS), args, SMEM_BYTES, st) != cudaSuccess)
-      return WK_E_CUDA;
+    if (int r = launch_pdl(k_resid, dim3(resid_count, a->Hq, a->B), THREADS, SMEM_BYTES, st, 1, {&tq, &tk, &tv, &p}))
+      return r;
+    p.first_in_call = 0;
   }
   if (num_m - main_first > 0) {
     p.m_first = main_first;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(num_m - main_first, a->Hq, a->B);
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = resid_count > 0 ? 1 : 0;
     // wide: one CTA per query block in the grid; the CTAs that start take over the blocks of those that have not yet
-    cfg.blockDim = dim3(wide ? M_THREADS : THREADS);
-    cfg.dynamicSmemBytes = wide ? M_SMEM_BYTES : SMEM_BYTES;
-    void* args[] = {&tq, wide ? &tk128 : &tk, wide ? &tv128 : &tv, &p};
-    if (cudaLaunchKernelExC(&cfg, wide ? k_wide : k_main, args) != cudaSuccess) return WK_E_CUDA;
+    if (int r = launch_pdl(wide ? k_wide : k_main, dim3(num_m - main_first, a->Hq, a->B), wide ? M_THREADS : THREADS,
+                                wide ? M_SMEM_BYTES : SMEM_BYTES, st, 1,
+                                {&tq, wide ? &tk128 : &tk, wide ? &tv128 : &tv, &p}))
+      return r;
   }
-  if (cudaGetLastError() != cudaSuccess) return WK_E_CUDA;
-  // blocks the kernels above flagged as beyond their exponent range are computed again (normally none)
-  return p.redo ? launch_attn_fwd_redo(a, false, p.redo, st) : 0;
+  return 0;
 }
 
 

@@ -530,3 +530,10 @@ int launch_attn_rows(const wk_attn_fwd_args* a, bool bf16, cudaStream_t stream) 
 }
 
 }  // namespace wk
+
+// One int per block of 128 queries, rounded up to 16 bytes.
+extern "C" int64_t wk_attn_fwd_workspace_bytes(int B, int Hq, int Nq) {
+  if (B <= 0 || Hq <= 0 || Nq <= 0) return 0;
+  const int64_t blocks = static_cast<int64_t>(B) * Hq * ((Nq + 127) / 128);
+  return (blocks * 4 + 15) / 16 * 16;
+}
