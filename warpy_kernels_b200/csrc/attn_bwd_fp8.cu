@@ -38,9 +38,11 @@
 #include <math.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 #include "host_common.h"
+#include "pair.cuh"
 
 namespace wk {
 namespace {
@@ -118,6 +120,8 @@ struct PrepParams {
 
 // one warp per query row, 4 consecutive elements per lane
 __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const PrepParams p) {
+  pdl_launch_dependents();  // the dK/dV kernel waits for this one to complete
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   const int64_t rows = static_cast<int64_t>(p.B) * p.Hq * p.nq_pad;
@@ -180,6 +184,8 @@ __global__ void __launch_bounds__(256) attn_bwd_prep_kernel(const PrepParams p) 
 // consecutive elements per lane, read with 16-byte loads (64 bytes in flight per thread instead of 16: the kernel is
 // HBM-bound and the one-row-per-warp form reached a third of the copy bandwidth).
 __global__ void __launch_bounds__(256) attn_bwd_prep4_kernel(const PrepParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   const int sub = lane & 7;
@@ -323,9 +329,64 @@ struct BwdParams {
   int B, Hq, Hkv, Nq, Nk, nq_pad;
   int d;  // head dimension, 128 or 64
   int causal;
+  int kv_splits, q_splits;  // CTAs of a cluster that share one key block (dK/dV) or query block (dQ)
   float softmax_scale;
   int* status;
 };
+
+// A small problem has fewer key or query blocks than the GPU has SMs.  Then the tiles of a block are divided among the
+// CTAs of a cluster, and the fp32 sums meet in distributed shared memory in chunks of 32 columns x 128 rows (16 KiB,
+// eight planes of 128 x 16 bytes): chunk i belongs to CTA i % splits, which adds the parts up in the order of the splits.
+// `recv` is shared memory that is idle in every CTA by then (the K / V and stage tiles).
+constexpr int X_CHUNK_BYTES = 128 * 32 * 4;
+__device__ __forceinline__ uint32_t exchange_slot(uint32_t recv, int splits, int chunks, int source, int owner, int chunk,
+                                                  int row) {
+  const int per_owner = (chunks + splits - 1) / splits;
+  return recv + static_cast<uint32_t>((source - (source > owner)) * per_owner + chunk / splits) * X_CHUNK_BYTES + row * 16;
+}
+__device__ __forceinline__ void exchange_send(uint32_t recv, int splits, int chunks, int me, int chunk, int row,
+                                              const uint32_t (&v)[32]) {
+  const int owner = chunk % splits;
+  const uint32_t dst = mapa(exchange_slot(recv, splits, chunks, me, owner, chunk, row), owner);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) st_cluster_v4(dst + j * (128 * 16), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+// v: this CTA's own part on entry, the sum over all splits on return.
+__device__ __forceinline__ void exchange_sum(uint32_t recv, int splits, int chunks, int me, int chunk, int row,
+                                             uint32_t (&v)[32]) {
+  float sum[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+#pragma unroll 1
+  for (int s = 0; s < splits; ++s) {
+    if (s == me) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) sum[i] += __uint_as_float(v[i]);
+      continue;
+    }
+    const uint32_t src = exchange_slot(recv, splits, chunks, s, me, chunk, row);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float4 x = lds_f4(src + j * (128 * 16));
+      sum[4 * j] += x.x, sum[4 * j + 1] += x.y, sum[4 * j + 2] += x.z, sum[4 * j + 3] += x.w;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(sum[i]);
+}
+// 32 values of a row, scaled, as bf16
+__device__ __forceinline__ void store_row32_bf16(__nv_bfloat16* dst_row, const uint32_t (&v)[32], float scale) {
+  uint4* dst = reinterpret_cast<uint4*>(dst_row);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    uint4 w;
+    w.x = pack_bf16x2(__uint_as_float(v[8 * i + 0]) * scale, __uint_as_float(v[8 * i + 1]) * scale);
+    w.y = pack_bf16x2(__uint_as_float(v[8 * i + 2]) * scale, __uint_as_float(v[8 * i + 3]) * scale);
+    w.z = pack_bf16x2(__uint_as_float(v[8 * i + 4]) * scale, __uint_as_float(v[8 * i + 5]) * scale);
+    w.w = pack_bf16x2(__uint_as_float(v[8 * i + 6]) * scale, __uint_as_float(v[8 * i + 7]) * scale);
+    dst[i] = w;
+  }
+}
 
 // ---------------------------------------------------------------------------
 // 2. dK / dV
@@ -350,7 +411,7 @@ constexpr int A_SF_COL = 192;   // per (h, k) 8 columns: the P scales in 0..3, t
 constexpr int A_SF_UNIT_COL = 224;  // scale 1 for the B operands, written once
 constexpr int A_DV_COL = 256, A_DK_COL = 384;
 
-template <int DH>
+template <int DH, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                      const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -424,27 +485,41 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  // What this kernel reads is there once the prep kernel has completed; the dQ kernel reads the same and may start from
+  // here on, beside this one (it ends after it).
+  pdl_wait();
+  pdl_launch_dependents();
 
   // The CTA's list of key blocks: its own grid index first, then the indices of CTAs that have not started, handed
   // out by the launch control (common.cuh) one at a time.  Tiles and blocks are counted through the CTA's whole life;
   // every barrier parity below derives from those running counts.
   struct KeyBlock {
     int n0, hkv, b, m_first, tiles_per_head, n_iter;
+    int it0;  // first of this CTA's iterations over the group's query heads and tiles
   } blk;
+  const int splits = SPLIT ? p.kv_splits : 1;
+  const int me = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
   auto set_block = [&](uint32_t x, uint32_t y, uint32_t z) {
-    blk.n0 = x * BN;
+    blk.n0 = (SPLIT ? x / splits : x) * BN;
     blk.hkv = y;
     blk.b = z;
     // first query tile that sees a key of this block (bottom-right aligned causal mask)
     blk.m_first = p.causal ? min(num_m, max(0, blk.n0 - shift) / BM) : 0;
     blk.tiles_per_head = num_m - blk.m_first;
     blk.n_iter = group * blk.tiles_per_head;
+    blk.it0 = 0;
+    if (SPLIT) {
+      const int all = blk.n_iter;
+      blk.it0 = all * me / splits;
+      blk.n_iter = all * (me + 1) / splits - blk.it0;
+    }
   };
   set_block(blockIdx.x, blockIdx.y, blockIdx.z);
   bool ok = true;
   uint32_t n_answers = 0;  // answers read so far
   // Reads the next answer of the launch control: false if no block was left (or the wait gave up: ok is false then).
   auto next_block = [&]() {
+    if (SPLIT) return false;
     const int slot = n_answers % SCHED_SLOTS;
     if (!mbar_wait(sched_full(slot), (n_answers / SCHED_SLOTS) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) {
       ok = false;
@@ -476,8 +551,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           for (int it = 0; it < blk.n_iter; ++it, ++gt) {
             const int s = gt % A_STAGES;
             const uint32_t ph = (gt / A_STAGES) & 1;
-            const int hq = blk.hkv * group + it / blk.tiles_per_head;
-            const int m0 = (blk.m_first + it % blk.tiles_per_head) * BM;
+            const int hq = blk.hkv * group + (blk.it0 + it) / blk.tiles_per_head;
+            const int m0 = (blk.m_first + (blk.it0 + it) % blk.tiles_per_head) * BM;
             if (!mbar_wait(q_empty(s), ph ^ 1, p.status, WK_ERR_TIMEOUT_EMPTY)) {
               ok = false;
               break;
@@ -492,6 +567,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
           if (!ok) break;
         }
+        if (SPLIT) break;
         // this block's loads are on their way: ask for another block
         const int slot = n_answers % SCHED_SLOTS;
         if (n_answers >= SCHED_SLOTS &&
@@ -653,7 +729,8 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const uint64_t sv2 = pack_f32x2(p.v_descale[sc], p.v_descale[sc]);
     if (n_iter > 0) ++ci;
 
-    int mt = blk.m_first;  // the query tile, restarting with every query head of the group
+    // the query tile, restarting with every query head of the group
+    int mt = blk.m_first + (n_iter > 0 ? blk.it0 % blk.tiles_per_head : 0);
     for (int it = 0; it < n_iter; ++it, ++g) {
       const int s = g % A_STAGES;
       const int m0 = mt * BM;
@@ -740,7 +817,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
     if (n_iter > 0 && ok) ok = mbar_wait_warp(acc_full, ci & 1, p.status, WK_ERR_TIMEOUT_MMA);
     PROBE(13);
-    if (ok) {
+    if (ok && !SPLIT) {
       tc_fence_after();
       const float dk_scale = p.softmax_scale * p.q_descale[sc];
       const int64_t row_off = ((static_cast<int64_t>(blk.b) * p.Hkv + blk.hkv) * p.Nk + key) * DH;
@@ -764,18 +841,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
             for (int i = 0; i < 32; ++i) v[i] = 0;
           }
-          if (key < p.Nk && c * 32 < DH) {
-            uint4* dst = reinterpret_cast<uint4*>(dst_row + c * 32);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint4 w;
-              w.x = pack_bf16x2(__uint_as_float(v[8 * i + 0]) * scale, __uint_as_float(v[8 * i + 1]) * scale);
-              w.y = pack_bf16x2(__uint_as_float(v[8 * i + 2]) * scale, __uint_as_float(v[8 * i + 3]) * scale);
-              w.z = pack_bf16x2(__uint_as_float(v[8 * i + 4]) * scale, __uint_as_float(v[8 * i + 5]) * scale);
-              w.w = pack_bf16x2(__uint_as_float(v[8 * i + 6]) * scale, __uint_as_float(v[8 * i + 7]) * scale);
-              dst[i] = w;
-            }
-          }
+          if (key < p.Nk && c * 32 < DH) store_row32_bf16(dst_row + c * 32, v, scale);
         }
       }
     }
@@ -785,6 +851,49 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
   }
   PROBE_FLUSH(0);
+  if (SPLIT) {
+    // chunks 0..3: dV, 4..7: dK; element-wise warp column c holds columns [32 c, 32 c + 32) of both
+    const int c = (warp - FIRST_EW_WARP) >> 2, row = (warp & 3) * 32 + lane;
+    const bool mine = warp >= FIRST_EW_WARP && c * 32 < DH;
+    const uint32_t acc = tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + c * 32;
+    auto part = [&](int which, uint32_t (&v)[32]) {
+      if (blk.n_iter > 0) {
+        tmem_ld32(acc + (which == 0 ? A_DV_COL : A_DK_COL), v);
+        tc_wait_ld();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = 0;
+      }
+    };
+    tc_fence_before();
+    __syncwarp();
+    cluster_sync();  // every CTA's products are complete: its tiles are idle
+    tc_fence_after();
+    if (mine) {
+#pragma unroll 1
+      for (int which = 0; which < 2; ++which) {
+        if ((4 * which + c) % splits == me) continue;
+        uint32_t v[32];
+        part(which, v);
+        exchange_send(smem_base, splits, 8, me, 4 * which + c, row, v);
+      }
+    }
+    __syncwarp();
+    cluster_sync();
+    if (mine) {
+      const int key = blk.n0 + row;
+      const int64_t row_off = ((static_cast<int64_t>(blk.b) * p.Hkv + blk.hkv) * p.Nk + key) * DH + c * 32;
+      const float dk_scale = p.softmax_scale * p.q_descale[blk.b * p.Hkv + blk.hkv];
+#pragma unroll 1
+      for (int which = 0; which < 2; ++which) {
+        if ((4 * which + c) % splits != me) continue;
+        uint32_t v[32];
+        part(which, v);
+        exchange_sum(smem_base, splits, 8, me, 4 * which + c, row, v);
+        if (key < p.Nk) store_row32_bf16((which == 0 ? p.dv : p.dk) + row_off, v, which == 0 ? 1.f : dk_scale);
+      }
+    }
+  }
 
   tc_fence_before();
   __syncthreads();
@@ -810,7 +919,7 @@ constexpr int B_SF_COL = 448;       // their scales: per tile buffer 16 columns,
 constexpr int B_SF_UNIT_COL = 480;  // scale 1 for the B operand, written once
 constexpr int EW_THREADS = 2 * HALF_THREADS;
 
-template <int DH>
+template <int DH, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -882,6 +991,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   PROBE(20);
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  // The dK/dV kernel lets this one start once the prep kernel, whose results both read, has completed: no wait here.
+  pdl_launch_dependents();
 
   // The CTA's list of query blocks: its own grid index first, then the indices of CTAs that have not started, handed
   // out by the launch control (common.cuh) one at a time, in launch order (the blocks with the most key tiles
@@ -889,9 +1000,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   // those running counts.
   struct QueryBlock {
     int m0, hq, b, hkv, n_tiles;
+    int j0;  // first of this CTA's key tiles
   } blk;
+  const int splits = SPLIT ? p.q_splits : 1;
+  const int me = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
   auto set_block = [&](uint32_t x, uint32_t y, uint32_t z) {
-    blk.m0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(x)) * BM;
+    blk.m0 = SPLIT ? static_cast<int>((gridDim.x - 1 - x) / splits) * BM
+                        : (static_cast<int>(gridDim.x) - 1 - static_cast<int>(x)) * BM;
     blk.hq = y;
     blk.b = z;
     blk.hkv = blk.hq / group;
@@ -901,12 +1016,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       n = last_key < 0 ? 0 : min(n, last_key / BN + 1);
     }
     blk.n_tiles = n;
+    blk.j0 = 0;
+    if (SPLIT) {
+      blk.j0 = n * me / splits;
+      blk.n_tiles = n * (me + 1) / splits - blk.j0;
+    }
   };
   set_block(blockIdx.x, blockIdx.y, blockIdx.z);
   bool ok = true;
   uint32_t n_answers = 0;  // answers read so far
   // Reads the next answer of the launch control: false if no block was left (or the wait gave up: ok is false then).
   auto next_block = [&]() {
+    if (SPLIT) return false;
     const int slot = n_answers % SCHED_SLOTS;
     if (!mbar_wait(sched_full(slot), (n_answers / SCHED_SLOTS) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) {
       ok = false;
@@ -944,11 +1065,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             }
             const uint32_t base = stage_smem + s * B_STAGE_BYTES;
             mbar_expect_tx(kv_full(s), B_STAGE_BYTES);
-            tma_load_4d(base, &tmap_k, kv_full(s), 0, j * BN, blk.hkv, blk.b);
-            tma_load_4d(base + TILE_BYTES, &tmap_v, kv_full(s), 0, j * BN, blk.hkv, blk.b);
+            tma_load_4d(base, &tmap_k, kv_full(s), 0, (blk.j0 + j) * BN, blk.hkv, blk.b);
+            tma_load_4d(base + TILE_BYTES, &tmap_v, kv_full(s), 0, (blk.j0 + j) * BN, blk.hkv, blk.b);
           }
           if (!ok) break;
         }
+        if (SPLIT) break;
         // this block's loads are on their way: ask for another block
         const int slot = n_answers % SCHED_SLOTS;
         if (n_answers >= SCHED_SLOTS &&
@@ -1084,7 +1206,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     uint32_t jt = 0;  // tiles so far
 
     for (;;) {
-    const int m0 = blk.m0, n_tiles = blk.n_tiles, hq = blk.hq, b = blk.b;
+    const int m0 = blk.m0, n_tiles = blk.n_tiles, hq = blk.hq, b = blk.b, key_base = blk.j0 * BN;
     const int row = m0 + r;
     const int sc = b * p.Hkv + blk.hkv;
     const float sq = p.q_descale[sc], sk = p.k_descale[sc];
@@ -1092,7 +1214,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const float* rec = p.qstat + ((static_cast<int64_t>(b) * p.Hq + hq) * p.nq_pad + m0) * 2 + r;
     const float neg_l = rec[0], neg_d = rec[128];  // log2(g) - L and -sum(dO8 . O) of this query
     const float gsv = p.v_descale[sc];  // dP = sv . dP8 in units of g
-    const int row_limit = min(p.causal ? row + shift : p.Nk - 1, p.Nk - 1);
+    const int row_limit = min(p.causal ? row + shift : p.Nk - 1, p.Nk - 1) - key_base;
     if (n_tiles > 0) ++ci;
 
     for (int j = 0; j < n_tiles; ++j, ++jt) {
@@ -1104,7 +1226,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       tc_fence_after();
       const int limit = row_limit - j * BN;  // columns > limit are masked
       // uniform over the CTA: does this tile contain any masked score?
-      const bool tile_masked = (j * BN + BN > p.Nk) || (p.causal && j * BN + BN - 1 > m0 + shift);
+      const bool tile_masked =
+          (key_base + j * BN + BN > p.Nk) || (p.causal && key_base + j * BN + BN - 1 > m0 + shift);
       uint32_t sf_d;
       {
         uint32_t sraw[32], draw[32];
@@ -1154,7 +1277,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 
     if (n_tiles > 0 && ok) ok = mbar_wait_warp(acc_full, ci & 1, p.status, WK_ERR_TIMEOUT_MMA);
     PROBE(13);
-    if (ok) {
+    if (ok && !SPLIT) {
       tc_fence_after();
       const float scale = p.softmax_scale * sk;
       __nv_bfloat16* dst_row = p.dq + ((static_cast<int64_t>(b) * p.Hq + hq) * p.Nq + row) * DH;
@@ -1171,23 +1294,45 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
-        if (row < p.Nq && c * 32 < DH) {
-          uint4* dst = reinterpret_cast<uint4*>(dst_row + c * 32);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint4 w;
-            w.x = pack_bf16x2(__uint_as_float(v[8 * i + 0]) * scale, __uint_as_float(v[8 * i + 1]) * scale);
-            w.y = pack_bf16x2(__uint_as_float(v[8 * i + 2]) * scale, __uint_as_float(v[8 * i + 3]) * scale);
-            w.z = pack_bf16x2(__uint_as_float(v[8 * i + 4]) * scale, __uint_as_float(v[8 * i + 5]) * scale);
-            w.w = pack_bf16x2(__uint_as_float(v[8 * i + 6]) * scale, __uint_as_float(v[8 * i + 7]) * scale);
-            dst[i] = w;
-          }
-        }
+        if (row < p.Nq && c * 32 < DH) store_row32_bf16(dst_row + c * 32, v, scale);
       }
     }
     PROBE(14);
     PROBE_COUNT(21);
     if (!ok || !next_block()) break;
+    }
+  }
+
+  if (SPLIT) {
+    const int c = (warp - FIRST_EW_WARP) >> 2, row = (warp & 3) * 32 + lane;
+    const bool mine = warp >= FIRST_EW_WARP && c * 32 < DH;
+    auto part = [&](uint32_t (&v)[32]) {
+      if (blk.n_tiles > 0) {
+        tmem_ld32(tmem_base + (static_cast<uint32_t>((warp & 3) * 32) << 16) + B_DQ_COL + c * 32, v);
+        tc_wait_ld();
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = 0;
+      }
+    };
+    tc_fence_before();
+    __syncwarp();
+    cluster_sync();  // every CTA's products are complete: its tiles are idle
+    tc_fence_after();
+    if (mine && c % splits != me) {
+      uint32_t v[32];
+      part(v);
+      exchange_send(smem_base, splits, 4, me, c, row, v);
+    }
+    __syncwarp();
+    cluster_sync();
+    if (mine && c % splits == me) {
+      uint32_t v[32];
+      part(v);
+      exchange_sum(smem_base, splits, 4, me, c, row, v);
+      if (blk.m0 + row < p.Nq)
+        store_row32_bf16(p.dq + ((static_cast<int64_t>(blk.b) * p.Hq + blk.hq) * p.Nq + blk.m0 + row) * DH + c * 32, v,
+                         p.softmax_scale * p.k_descale[blk.b * p.Hkv + blk.hkv]);
     }
   }
 
@@ -1198,6 +1343,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
   PROBE_FLUSH(24);
+  pdl_wait();  // does not end before the dK/dV kernel has
 }
 
 // Rows of `d` bytes under boxes of 128: with head dimension 64 TMA fills the upper half of every row with zeros.
@@ -1207,6 +1353,35 @@ int make_map4(CUtensorMap* m, const void* base, int d, int n, int h, int b, cons
                            static_cast<uint64_t>(strides[0])};
   const uint32_t box[4] = {D, 128, 1, 1};
   return encode_tmap(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, base, dims, str, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// How many CTAs share a key block and a query block.  The two kernels run side by side when their CTAs fit the SMs
+// together (clusters do not use all of them: about nine tenths).  Cycles as the model has them: 3000 per 128 x 128 tile
+// of the dK/dV kernel and 2000 of the dQ kernel, start and end of a CTA 8000 and 6000, the exchange 5000.
+void bwd_splits(const wk_attn_bwd_args* a, int num_n, int num_m, int sms, int& kv, int& q) {
+  kv = q = 1;
+  const int64_t kv_units = static_cast<int64_t>(num_n) * a->Hkv * a->B, q_units = static_cast<int64_t>(num_m) * a->Hq * a->B;
+  const int kv_tiles = num_m * (a->Hq / a->Hkv), q_tiles = num_n;
+  const int fit = sms * 9 / 10;
+  if (kv_units > fit / 2 && q_units > fit / 2) return;
+  auto rounds = [&](int64_t ctas) { return static_cast<double>((ctas + sms - 1) / sms); };
+  double best = 1e30;
+  static const int kSplits[] = {1, 2, 3, 4, 6, 8};
+  for (int sk : kSplits) {
+    if (sk > 1 && (kv_units * sk > fit || sk > kv_tiles)) continue;
+    for (int sq : kSplits) {
+      if (sq > 1 && (q_units * sq > fit || sq > q_tiles)) continue;
+      const double t_kv = rounds(kv_units * sk) * (8000 + (sk > 1 ? 5000 : 0) + (kv_tiles + sk - 1) / sk * 3000.0);
+      const double t_q = rounds(q_units * sq) * (6000 + (sq > 1 ? 5000 : 0) + (q_tiles + sq - 1) / sq * 2000.0);
+      const bool together = kv_units * sk + q_units * sq <= (sk > 1 || sq > 1 ? fit : sms);
+      const double t = (together ? (t_kv > t_q ? t_kv : t_q) : t_kv + t_q) + 10.0 * (sk + sq);
+      if (t < best) {
+        best = t;
+        kv = sk;
+        q = sq;
+      }
+    }
+  }
 }
 
 }  // namespace
@@ -1294,13 +1469,10 @@ extern "C" int wk_attn_bwd_fp8(const wk_attn_bwd_args* a, void* stream) {
     const int64_t rows = static_cast<int64_t>(a->B) * a->Hq * nq_pad;
     bool wide_loads = aligned16(a->out) && aligned16(a->dout);  // 16-byte loads: rows on 16-byte boundaries
     for (int i = 0; i < 3; ++i) wide_loads = wide_loads && a->out_strides[i] % 8 == 0 && a->dout_strides[i] % 8 == 0;
-    if (wide_loads) {
-      attn_bwd_prep4_kernel<<<static_cast<unsigned>((rows + 31) / 32), 256, 0, st>>>(pp);
-    } else {
-      const int64_t blocks = (rows + 7) / 8;
-      attn_bwd_prep_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(pp);
-    }
-    if (cudaGetLastError() != cudaSuccess) return WK_E_CUDA;
+    const void* kernel = wide_loads ? reinterpret_cast<const void*>(attn_bwd_prep4_kernel)
+                                    : reinterpret_cast<const void*>(attn_bwd_prep_kernel);
+    const int64_t blocks = wide_loads ? (rows + 31) / 32 : (rows + 7) / 8;
+    if (int r = launch_pdl(kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, st, 1, {&pp})) return r;
   }
 
   CUtensorMap tq, tk, tv, tdo;
@@ -1333,19 +1505,22 @@ extern "C" int wk_attn_bwd_fp8(const wk_attn_bwd_args* a, void* stream) {
   p.softmax_scale = a->softmax_scale;
   p.status = status;
 
-  if (allow_smem((a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<128>)), A_SMEM_BYTES)) return WK_E_CUDA;
-  if (allow_smem((a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_dq_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_dq_kernel<128>)), B_SMEM_BYTES)) return WK_E_CUDA;
-  {
-    dim3 grid((a->Nk + BN - 1) / BN, a->Hkv, a->B);
-    void* args[] = {&tq, &tk, &tv, &tdo, &p};
-    const void* kernel = a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_dkdv_kernel<128>);
-    if (cudaLaunchKernel(kernel, grid, dim3(THREADS), args, A_SMEM_BYTES, st) != cudaSuccess) return WK_E_CUDA;
-  }
-  {
-    dim3 grid((a->Nq + BM - 1) / BM, a->Hq, a->B);
-    void* args[] = {&tq, &tk, &tv, &tdo, &p};
-    const void* kernel = a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_dq_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_dq_kernel<128>);
-    if (cudaLaunchKernel(kernel, grid, dim3(THREADS), args, B_SMEM_BYTES, st) != cudaSuccess) return WK_E_CUDA;
-  }
-  return 0;
+  const int sms = sm_count();
+  if (sms <= 0) return WK_E_CUDA;
+  const int num_n = (a->Nk + BN - 1) / BN, num_m = (a->Nq + BM - 1) / BM;
+  bwd_splits(a, num_n, num_m, sms, p.kv_splits, p.q_splits);
+  auto pick = [&](auto... forms) {  // [head dimension 128 / 64][whole / split]
+    const void* f[] = {reinterpret_cast<const void*>(forms)...};
+    return std::make_pair(f[2 * (a->d == 64) + (p.kv_splits > 1)], f[4 + 2 * (a->d == 64) + (p.q_splits > 1)]);
+  };
+  const auto [dkdv, dq] = pick(attn_bwd_dkdv_kernel<128, false>, attn_bwd_dkdv_kernel<128, true>,
+                               attn_bwd_dkdv_kernel<64, false>, attn_bwd_dkdv_kernel<64, true>,
+                               attn_bwd_dq_kernel<128, false>, attn_bwd_dq_kernel<128, true>,
+                               attn_bwd_dq_kernel<64, false>, attn_bwd_dq_kernel<64, true>);
+  if (allow_smem(dkdv, A_SMEM_BYTES) || allow_smem(dq, B_SMEM_BYTES)) return WK_E_CUDA;
+  if ((r = launch_pdl(dkdv, dim3(num_n * p.kv_splits, a->Hkv, a->B), THREADS, A_SMEM_BYTES, st, p.kv_splits,
+                      {&tq, &tk, &tv, &tdo, &p})))
+    return r;
+  return launch_pdl(dq, dim3(num_m * p.q_splits, a->Hq, a->B), THREADS, B_SMEM_BYTES, st, p.q_splits,
+                    {&tq, &tk, &tv, &tdo, &p});
 }
