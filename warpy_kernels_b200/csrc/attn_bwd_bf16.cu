@@ -56,6 +56,8 @@ struct PrepParams {
 
 // one warp per query row, 4 consecutive elements per lane
 __global__ void __launch_bounds__(256) attn_bwd_bf16_prep_kernel(const PrepParams p) {
+  pdl_launch_dependents();  // the dK/dV kernel waits for this one to complete
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   const int64_t rows = static_cast<int64_t>(p.B) * p.Hq * p.nq_pad;
@@ -91,6 +93,8 @@ __global__ void __launch_bounds__(256) attn_bwd_bf16_prep_kernel(const PrepParam
 // consecutive elements per lane, read with 16-byte loads (the kernel is HBM-bound; one row per warp keeps too few
 // bytes in flight).
 __global__ void __launch_bounds__(256) attn_bwd_bf16_prep4_kernel(const PrepParams p) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
   const int sub = lane & 7;
@@ -166,6 +170,7 @@ struct BwdParams {
   int B, Hq, Hkv, Nq, Nk, nq_pad;
   int d;  // head dimension, 128 or 64
   int causal;
+  int kv_band, q_band;  // heads whose blocks are handed out together (band_order)
   float softmax_scale;
   int* status;
 };
@@ -202,10 +207,10 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
 
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
-  const int n_blk = blockIdx.x;
-  const int hkv = blockIdx.y;
-  const int b = blockIdx.z;
-  const int n0 = n_blk * BN;
+  const BandBlock at = band_order(blockIdx.x, (p.Nk + BN - 1) / BN, p.B * p.Hkv, p.kv_band);
+  const int hkv = at.head % p.Hkv;
+  const int b = at.head / p.Hkv;
+  const int n0 = at.rank * BN;  // the first key blocks see the most queries
   const int group = p.Hq / p.Hkv;
   const int shift = p.Nk - p.Nq;
   const int num_m = (p.Nq + BM - 1) / BM;
@@ -240,6 +245,10 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  // What this kernel reads is there once the prep kernel has completed; the dQ kernel reads the same and may start from
+  // here on, beside this one (it ends after it).
+  pdl_wait();
+  pdl_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0 && n_iter > 0) {
@@ -493,11 +502,12 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
-  const int m_blk = gridDim.x - 1 - blockIdx.x;
-  const int hq = blockIdx.y;
-  const int b = blockIdx.z;
+  const int num_m = (p.Nq + BM - 1) / BM;
+  const BandBlock at = band_order(blockIdx.x, num_m, p.B * p.Hq, p.q_band);
+  const int hq = at.head % p.Hq;
+  const int b = at.head / p.Hq;
   const int hkv = hq / (p.Hq / p.Hkv);
-  const int m0 = m_blk * BM;
+  const int m0 = (num_m - 1 - at.rank) * BM;  // the last query blocks see the most keys
   const int shift = p.Nk - p.Nq;
   int n_tiles = (p.Nk + BN - 1) / BN;
   if (p.causal) {
@@ -531,6 +541,7 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  pdl_launch_dependents();
 
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
@@ -707,6 +718,7 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
+  if (blockIdx.x == gridDim.x - 1) pdl_wait();  // this kernel does not end before the dK/dV kernel has
 }
 
 int make_map4(CUtensorMap* m, const void* base, int d, int n, int h, int b, const int64_t* strides) {
@@ -775,13 +787,10 @@ extern "C" int wk_attn_bwd_bf16(const wk_attn_bwd_args* a, void* stream) {
     const int64_t rows = static_cast<int64_t>(a->B) * a->Hq * nq_pad;
     bool wide_loads = aligned16(a->out) && aligned16(a->dout);  // 16-byte loads: rows on 16-byte boundaries
     for (int i = 0; i < 3; ++i) wide_loads = wide_loads && a->out_strides[i] % 8 == 0 && a->dout_strides[i] % 8 == 0;
-    if (wide_loads) {
-      attn_bwd_bf16_prep4_kernel<<<static_cast<unsigned>((rows + 31) / 32), 256, 0, st>>>(pp);
-    } else {
-      const int64_t blocks = (rows + 7) / 8;
-      attn_bwd_bf16_prep_kernel<<<static_cast<unsigned>(blocks), 256, 0, st>>>(pp);
-    }
-    if (cudaGetLastError() != cudaSuccess) return WK_E_CUDA;
+    const void* kernel = wide_loads ? reinterpret_cast<const void*>(attn_bwd_bf16_prep4_kernel)
+                                    : reinterpret_cast<const void*>(attn_bwd_bf16_prep_kernel);
+    const int64_t blocks = wide_loads ? (rows + 31) / 32 : (rows + 7) / 8;
+    if (int r = launch_pdl(kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, st, 1, {&pp})) return r;
   }
 
   CUtensorMap tq, tk, tv, tdo;
@@ -810,19 +819,23 @@ extern "C" int wk_attn_bwd_bf16(const wk_attn_bwd_args* a, void* stream) {
   p.softmax_scale = a->softmax_scale;
   p.status = status;
 
-  if (allow_smem((a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_bf16_dkdv_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_bf16_dkdv_kernel<128>)), A_SMEM_BYTES)) return WK_E_CUDA;
-  if (allow_smem((a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_bf16_dq_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_bf16_dq_kernel<128>)), B_SMEM_BYTES)) return WK_E_CUDA;
-  {
-    dim3 grid((a->Nk + BN - 1) / BN, a->Hkv, a->B);
-    void* args[] = {&tq, &tk, &tv, &tdo, &p};
-    const void* kernel = a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_bf16_dkdv_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_bf16_dkdv_kernel<128>);
-    if (cudaLaunchKernel(kernel, grid, dim3(THREADS), args, A_SMEM_BYTES, st) != cudaSuccess) return WK_E_CUDA;
-  }
-  {
-    dim3 grid((a->Nq + BM - 1) / BM, a->Hq, a->B);
-    void* args[] = {&tq, &tk, &tv, &tdo, &p};
-    const void* kernel = a->d == 64 ? reinterpret_cast<const void*>(attn_bwd_bf16_dq_kernel<64>) : reinterpret_cast<const void*>(attn_bwd_bf16_dq_kernel<128>);
-    if (cudaLaunchKernel(kernel, grid, dim3(THREADS), args, B_SMEM_BYTES, st) != cudaSuccess) return WK_E_CUDA;
-  }
-  return 0;
+  const int num_n = (a->Nk + BN - 1) / BN, num_m = nq_pad / BM;
+  const int sms = sm_count();
+  if (sms <= 0) return WK_E_CUDA;
+  // q, dO, k and v of a KV head
+  const int group = a->Hq / a->Hkv;
+  const int64_t head_bytes = 4ll * a->d * (static_cast<int64_t>(group) * a->Nq + a->Nk);
+  p.kv_band = a->causal ? band_heads(num_n, a->B * a->Hkv, head_bytes, sms) : 1;
+  p.q_band = a->causal ? band_heads(num_m, a->B * a->Hq, head_bytes / group, sms) : 1;
+  const bool small = a->d == 64;
+  const void* dkdv = small ? reinterpret_cast<const void*>(attn_bwd_bf16_dkdv_kernel<64>)
+                           : reinterpret_cast<const void*>(attn_bwd_bf16_dkdv_kernel<128>);
+  const void* dq = small ? reinterpret_cast<const void*>(attn_bwd_bf16_dq_kernel<64>)
+                         : reinterpret_cast<const void*>(attn_bwd_bf16_dq_kernel<128>);
+  if (allow_smem(dkdv, A_SMEM_BYTES) || allow_smem(dq, B_SMEM_BYTES)) return WK_E_CUDA;
+  const int64_t kv_ctas = static_cast<int64_t>(num_n) * a->Hkv * a->B, q_ctas = static_cast<int64_t>(num_m) * a->Hq * a->B;
+  if (kv_ctas > INT32_MAX || q_ctas > INT32_MAX) return WK_E_ARG;
+  if ((r = launch_pdl(dkdv, dim3(static_cast<unsigned>(kv_ctas)), THREADS, A_SMEM_BYTES, st, 1, {&tq, &tk, &tv, &tdo, &p})))
+    return r;
+  return launch_pdl(dq, dim3(static_cast<unsigned>(q_ctas)), THREADS, B_SMEM_BYTES, st, 1, {&tq, &tk, &tv, &tdo, &p});
 }

@@ -144,6 +144,21 @@ __device__ __forceinline__ void pdl_launch_dependents() {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
+// Which block of an attention problem a CTA takes.  Under the causal mask the blocks of a head differ by up to its
+// number of tiles, and CTAs start in the order of their index: blocks go out longest first over a band of heads (rank 0
+// is the longest block of each head of the band), see band_heads().
+// ---------------------------------------------------------------------------
+struct BandBlock {
+  int rank, head;
+};
+__device__ __forceinline__ BandBlock band_order(uint32_t id, int blocks, int heads, int band) {
+  const uint32_t full = static_cast<uint32_t>(band) * blocks;
+  const int first = static_cast<int>(id / full) * band;
+  const uint32_t in_band = id % full, width = min(band, heads - first);
+  return {static_cast<int>(in_band / width), first + static_cast<int>(in_band % width)};
+}
+
+// ---------------------------------------------------------------------------
 // Launch control: a running CTA takes over the grid index of a CTA that has not started yet, so that a grid with
 // one CTA per work item is worked through by the CTAs that fit the GPU, in launch order, without the start-up and
 // drain of a CTA between items.  After an answer that says "none left" no further request may be made.
