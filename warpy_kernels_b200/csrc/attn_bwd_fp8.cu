@@ -329,6 +329,7 @@ struct BwdParams {
   int B, Hq, Hkv, Nq, Nk, nq_pad;
   int d;  // head dimension, 128 or 64
   int causal;
+  int kv_band, q_band;      // heads whose blocks are handed out together (band_heads)
   int kv_splits, q_splits;  // CTAs of a cluster that share one key block (dK/dV) or query block (dQ)
   float softmax_scale;
   int* status;
@@ -500,6 +501,7 @@ attn_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int splits = SPLIT ? p.kv_splits : 1;
   const int me = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
   auto set_block = [&](uint32_t x, uint32_t y, uint32_t z) {
+    if (!SPLIT) band_order_grid(x, y, z, p.kv_band);
     blk.n0 = (SPLIT ? x / splits : x) * BN;
     blk.hkv = y;
     blk.b = z;
@@ -1005,6 +1007,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   const int splits = SPLIT ? p.q_splits : 1;
   const int me = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
   auto set_block = [&](uint32_t x, uint32_t y, uint32_t z) {
+    if (!SPLIT) band_order_grid(x, y, z, p.q_band);
     blk.m0 = SPLIT ? static_cast<int>((gridDim.x - 1 - x) / splits) * BM
                         : (static_cast<int>(gridDim.x) - 1 - static_cast<int>(x)) * BM;
     blk.hq = y;
@@ -1509,6 +1512,11 @@ extern "C" int wk_attn_bwd_fp8(const wk_attn_bwd_args* a, void* stream) {
   if (sms <= 0) return WK_E_CUDA;
   const int num_n = (a->Nk + BN - 1) / BN, num_m = (a->Nq + BM - 1) / BM;
   bwd_splits(a, num_n, num_m, sms, p.kv_splits, p.q_splits);
+  // q, dO8, k and v of a KV head
+  const int group = a->Hq / a->Hkv;
+  const int64_t head_bytes = 2ll * a->d * (static_cast<int64_t>(group) * a->Nq + a->Nk);
+  p.kv_band = a->causal ? band_heads(num_n, a->B * a->Hkv, head_bytes, sms) : 1;
+  p.q_band = a->causal ? band_heads(num_m, a->B * a->Hq, head_bytes / group, sms) : 1;
   auto pick = [&](auto... forms) {  // [head dimension 128 / 64][whole / split]
     const void* f[] = {reinterpret_cast<const void*>(forms)...};
     return std::make_pair(f[2 * (a->d == 64) + (p.kv_splits > 1)], f[4 + 2 * (a->d == 64) + (p.q_splits > 1)]);

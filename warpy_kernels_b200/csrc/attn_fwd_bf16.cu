@@ -64,7 +64,7 @@ struct FwdParams {
   int lse_natural;
   const int* seqused_k;  // [B] or null
   float softmax_scale;
-  int m_first;  // first query block of this launch (the grid covers gridDim.x blocks from here)
+  int band;  // heads whose blocks are handed out together (band_heads)
   int* status;
   ExactInputs exact;  // rows whose scores outgrow the row reference
 };
@@ -138,9 +138,11 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
   pdl_wait();
-  const int m_blk = p.m_first + gridDim.x - 1 - blockIdx.x;  // longest (latest) causal blocks first
-  const int hq = blockIdx.y;
-  const int b = blockIdx.z;
+  uint32_t bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
+  band_order_grid(bx, by, bz, p.band);
+  const int m_blk = gridDim.x - 1 - bx;  // longest (latest) causal blocks first
+  const int hq = by;
+  const int b = bz;
   const int hkv = hq / (p.Hq / p.Hkv);
   const int m0 = m_blk * BM;
   // keys this batch item attends to; the causal diagonal is aligned to that length
@@ -491,7 +493,11 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
                                   : reinterpret_cast<const void*>(attn_fwd_bf16_kernel<128>);
   if (allow_smem(kernel, SMEM_BYTES)) return WK_E_CUDA;
   const int num_m = (a->Nq + BM - 1) / BM;
-  p.m_first = 0;
+  const int sms = sm_count();
+  if (sms <= 0) return WK_E_CUDA;
+  // q, out and a share of k and v
+  const int64_t head_bytes = 4ll * a->d * (a->Nq + static_cast<int64_t>(a->Nk) * a->Hkv / a->Hq);
+  p.band = a->causal ? band_heads(num_m, a->B * a->Hq, head_bytes, sms) : 1;
   return launch_pdl(kernel, dim3(num_m, a->Hq, a->B), THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream), 1,
                     {&tq, &tk, &tv, &p});
 }

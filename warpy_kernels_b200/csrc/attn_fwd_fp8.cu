@@ -120,6 +120,7 @@ struct FwdParams {
   const int* seqused_k;  // [B] or null
   float softmax_scale;
   int m_first;  // first query block of this launch (the grid covers gridDim.x blocks from here)
+  int band;     // heads whose blocks are handed out together (band_heads)
   int* status;
   int first_in_call;  // no kernel of this call before this one: wait for the stream's earlier work
   ExactInputs exact;  // rows whose scores outgrow the row reference
@@ -205,9 +206,11 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
   if (p.first_in_call) pdl_wait();
-  const int m_blk = p.m_first + gridDim.x - 1 - blockIdx.x;  // longest (latest) causal blocks first
-  const int hq = blockIdx.y;
-  const int b = blockIdx.z;
+  uint32_t bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
+  band_order_grid(bx, by, bz, p.band);
+  const int m_blk = p.m_first + gridDim.x - 1 - bx;  // longest (latest) causal blocks first
+  const int hq = by;
+  const int b = bz;
   const int hkv = hq / (p.Hq / p.Hkv);
   const int m0 = m_blk * BM;
   // keys this batch item attends to; the causal diagonal is aligned to that length
@@ -553,6 +556,7 @@ constexpr int M_CONSUMERS = 3 + M_SOFTMAX_THREADS;  // threads that read every a
 
 // The query block of grid index (x, y, z); false if it belongs to the two-term variant's launch.
 __device__ __forceinline__ bool wide_item(const FwdParams& p, uint32_t x, uint32_t y, uint32_t z, WideItem& it) {
+  band_order_grid(x, y, z, p.band);
   const int m_blk = p.m_first + gridDim.x - 1 - x;  // longest (latest) causal blocks first
   it.hq = y;
   it.b = z;
@@ -1239,12 +1243,16 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   p.first_in_call = 1;
   if (resid_count > 0) {
     p.m_first = 0;
+    p.band = 1;  // blocks of few tiles
     if (int r = launch_pdl(k_resid, dim3(resid_count, a->Hq, a->B), THREADS, SMEM_BYTES, st, 1, {&tq, &tk, &tv, &p}))
       return r;
     p.first_in_call = 0;
   }
   if (num_m - main_first > 0) {
     p.m_first = main_first;
+    // q, out and a share of k and v
+    const int64_t head_bytes = a->d * (3ll * a->Nq + 2ll * a->Nk * a->Hkv / a->Hq);
+    p.band = a->causal ? band_heads(num_m - main_first, a->B * a->Hq, head_bytes, sms) : 1;
     // wide: one CTA per query block in the grid; the CTAs that start take over the blocks of those that have not yet
     if (int r = launch_pdl(wide ? k_wide : k_main, dim3(num_m - main_first, a->Hq, a->B), wide ? M_THREADS : THREADS,
                                 wide ? M_SMEM_BYTES : SMEM_BYTES, st, 1,

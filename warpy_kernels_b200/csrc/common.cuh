@@ -157,6 +157,15 @@ __device__ __forceinline__ BandBlock band_order(uint32_t id, int blocks, int hea
   const uint32_t in_band = id % full, width = min(band, heads - first);
   return {static_cast<int>(in_band / width), first + static_cast<int>(in_band % width)};
 }
+// The same for a grid (blocks, heads, batch items) whose x counts from the longest block on.
+__device__ __forceinline__ void band_order_grid(uint32_t& x, uint32_t& y, uint32_t& z, int band) {
+  if (band > 1) {
+    const BandBlock at = band_order(x + gridDim.x * (y + gridDim.y * z), gridDim.x, gridDim.y * gridDim.z, band);
+    x = at.rank;
+    y = at.head % gridDim.y;
+    z = at.head / gridDim.y;
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Launch control: a running CTA takes over the grid index of a CTA that has not started yet, so that a grid with

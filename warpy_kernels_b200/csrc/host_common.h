@@ -46,7 +46,8 @@ int launch_pdl(const void* func, dim3 grid, int threads, int smem, cudaStream_t 
 // KV heads of 16 key blocks take 102 tile times on 148 SMs where 60 are work, longest first over all of them 65.  That is
 // only worth anything where CTAs are few per SM (at eight it is 3 % at most, and neighbours in time no longer share a head's
 // tensors), and the heads of a band have to fit L2 together.  BF16 backward: 2 x 32 heads, 2048 x 2048 290 -> 279 us,
-// 2 x 16 heads, d 64 130 -> 121, 4 heads, 12000 x 3000 82 -> 65; but 4 x 32 heads, 4096 x 4096 2200 -> 2236.
+// 2 x 16 heads, d 64 130 -> 121, 4 heads, 12000 x 3000 82 -> 65; but 4 x 32 heads, 4096 x 4096 2200 -> 2236.  Forward: BF16, 2 x 32 heads,
+// 2048 x 2048 102 -> 88 us, 16 heads, 4096 x 4096 127 -> 97 (FP8 81 -> 70).
 inline int band_heads(int blocks, int heads, int64_t head_bytes, int sms) {
   if (static_cast<int64_t>(blocks) * heads > 8ll * sms) return 1;
   const int64_t fit = (96ll << 20) / (head_bytes > 0 ? head_bytes : 1);
