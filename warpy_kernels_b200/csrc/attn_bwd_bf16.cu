@@ -7,18 +7,25 @@
 // kernels and the same pipeline as the FP8 backward (attn_bwd_fp8.cu), with tcgen05.mma kind::f16 and P^T, dS^T
 // rounded to bf16 instead of MXFP8:
 //
-//  1. attn_bwd_prep_kernel: per query row D = sum(dO . O) and the row record (-L, -D).
-//  2. attn_bwd_dkdv_kernel: CTA = 128 keys of one (batch, kv head), K and V resident in shared memory, loop over
+//  1. attn_bwd_bf16_prep4_kernel (attn_bwd_bf16_prep_kernel for rows not on 16-byte boundaries): per query row
+//     D = sum(dO . O) and the row record (-L, -D).
+//  2. attn_bwd_bf16_dkdv_kernel: CTA = 128 keys of one (batch, kv head), K and V resident in shared memory, loop over
 //     the group's query heads and query tiles; S^T = K Q^T and dP^T = V dO^T into TMEM, threads turn them into
 //     bf16 P^T and dS^T back in TMEM, dV += P^T dO and dK += dS^T Q (A from TMEM, B = the same Q / dO tiles read
 //     MN-major).  dV and dK stay in TMEM for the whole CTA.
-//  3. attn_bwd_dq_kernel: CTA = 128 queries, loop over key tiles, recomputes S and dP, dQ += dS K in TMEM: no
-//     atomics, deterministic.
+//  3. attn_bwd_bf16_dq_kernel: CTA = 128 queries, loop over key tiles, recomputes S and dP, dQ += dS K in TMEM: no
+//     atomics, deterministic.  It runs beside the dK/dV kernel.
 // A row of a tile is 256 bytes, two 128-byte swizzle spans: every tile is two boxes of 64 head-dim elements,
 // 16 KiB apart in shared memory.
 //
-// Tensor-core bound: 10 . B . Hq . Nq . Nk . d flops of algorithmic work (half when causal).
+// Tensor-core bound: 10 . B . Hq . Nq . Nk . d flops of algorithmic work (half when causal).  Per 128 x 128 tile the dQ
+// kernel takes 2180 cycles (1536 of tensor pipe), the dK/dV kernel 3600 (2560: its N = 64 products are paced by the
+// shared-memory reads of their operands); the chain from a score buffer's release to its next scores paces both.  With the
+// codes written over the scores and one thread issuing all products the two took 8600 cycles: 4 x 32 heads, 4096 x 4096
+// without mask 3966 -> 3491 us, causal 2235 -> 1953, 2 x 32 / 8 heads, 2048 x 2048 causal 278 -> 240.
 #include <math.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "host_common.h"
@@ -34,9 +41,9 @@ constexpr int CHUNK = 64;                        // head-dim elements per 128-by
 constexpr int CHUNK_BYTES = 128 * CHUNK * 2;     // 16 KiB: 128 rows x 128 bytes
 constexpr int TILE_BYTES = 2 * CHUNK_BYTES;      // 32 KiB: 128 rows x 256 bytes
 constexpr int SF_BYTES = 512;
-constexpr int THREADS = 576;          // TMA warp, MMA warp, 16 element-wise warps (four threads per row)
-constexpr int HALF_THREADS = 256;     // the element-wise threads of one 64-column half of a tile: two per row
-constexpr int HALF_COLS = 64;
+constexpr int THREADS = 640;        // TMA warp, three MMA warps, 16 element-wise warps (four threads per row of a tile)
+constexpr int EW_THREADS = 512;
+constexpr int GROUP_THREADS = 256;  // dK/dV: the element-wise threads of one 64-query half of a tile
 constexpr int TMEM_COLS = 512;
 constexpr float LOG2E = 1.4426950408889634f;
 
@@ -184,7 +191,10 @@ constexpr int A_STAGE_BYTES = 2 * TILE_BYTES + A_STAT_BYTES;
 // Requested size is padded past half an SM's shared memory: each CTA allocates all 512 TMEM columns, so a second
 // resident CTA could only spin in tcgen05.alloc.
 constexpr int A_SMEM_BYTES = 2 * TILE_BYTES + A_STAGES * A_STAGE_BYTES + 1024 + 256;  // 197 KiB: one CTA per SM
-constexpr int A_ST_COL = 0, A_DPT_COL = 128, A_DV_COL = 256, A_DK_COL = 384;
+// Work goes by units of 64 queries: S^T and dP^T of a unit go into the one score buffer, which the unit's element-wise
+// group (h = 0, 1 in turn) frees as soon as it holds the values in registers; P^T and dS^T go to columns of their own, one
+// set per group.  So the scores of the next unit are under way while a unit's P and dS are computed and its sums issued.
+constexpr int A_ST_COL = 0, A_DPT_COL = 64, A_P_COL = 128, A_DS_COL = 192, A_DV_COL = 256, A_DK_COL = 384;
 template <int DH>
 __global__ void __launch_bounds__(THREADS, 1)
 attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -199,10 +209,13 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   const uint32_t kv_full = bar_base;
   auto q_full = [&](int s) { return bar_base + 8u * (1 + s); };
   auto q_empty = [&](int s) { return bar_base + 8u * (1 + A_STAGES + s); };
-  // the two 64-query halves of a tile are handed back and forth separately (h = 0, 1)
-  auto s_full = [&](int h) { return bar_base + 8u * (1 + 2 * A_STAGES + h); };
-  auto p_full = [&](int h) { return bar_base + 8u * (3 + 2 * A_STAGES + h); };
-  const uint32_t acc_full = bar_base + 8u * (5 + 2 * A_STAGES);
+  // of the two element-wise groups (h = 0, 1)
+  const uint32_t misc = bar_base + 8u * (1 + 2 * A_STAGES);
+  auto s_full = [&](int h) { return misc + 8u * h; };
+  auto s_free = [&](int h) { return misc + 16 + 8u * h; };
+  auto p_full = [&](int h) { return misc + 32 + 8u * h; };  // the group's P^T and dS^T are in tensor memory
+  auto p_free = [&](int h) { return misc + 48 + 8u * h; };  // the products that read them are complete
+  const uint32_t acc_full = misc + 64;
   const uint32_t tmem_slot = acc_full + 8;
 
   const int warp = threadIdx.x / 32;
@@ -226,8 +239,10 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       mbar_init(q_empty(s), 1);
     }
     for (int h = 0; h < 2; ++h) {
-      mbar_init(s_full(h), 1);
-      mbar_init(p_full(h), HALF_THREADS);
+      mbar_init(s_full(h), 2);  // S^T and dP^T come from two threads
+      mbar_init(s_free(h), GROUP_THREADS);
+      mbar_init(p_full(h), GROUP_THREADS);
+      mbar_init(p_free(h), 1);
     }
     mbar_init(acc_full, 1);
     mbar_fence_init();
@@ -275,156 +290,131 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (warp == 1 || warp == 2) {
     if (lane == 0 && n_iter > 0) {
-      // A tile is processed as two halves of 64 queries, each with its own pair of barriers, so that the tensor
-      // pipe works on one half while the element-wise warps of the other half are busy:
-      //   S^T, dP^T (h) -> element-wise (h) -> dV, dK += (h) -> S^T, dP^T of the next tile (h) -> ...
-      // All MMAs come from this one thread, so the products of the next tile overwrite a half's columns only
-      // after the products that read its codes (the tensor pipe runs in issue order).
-      constexpr uint32_t idesc_ss = make_idesc(1, 1, 0, 0, BN, BM / 2);
-      const uint32_t idesc_ts = make_idesc(1, 1, 0, 1, BN, DH);  // B read MN-major, N = head dimension
-      const uint32_t st_tmem = tmem_base + A_ST_COL;
-      const uint32_t dpt_tmem = tmem_base + A_DPT_COL;
+      // S^T = K Q^T by warp 1, dP^T = V dO^T by warp 2, side by side: the time from the buffer's release to its next
+      // scores is on every unit's critical path, and a thread needs ~90 cycles per MMA it issues here
+      const int which = warp - 1;
+      constexpr uint32_t idesc = make_idesc(1, 1, 0, 0, BN, BM / 2);
+      const uint32_t d_tmem = tmem_base + (which == 0 ? A_ST_COL : A_DPT_COL);
+      const uint64_t a_desc = smem_desc_sw128(which == 0 ? k_smem : v_smem, 16, 1024);
       bool ok = mbar_wait(kv_full, 0, p.status, WK_ERR_TIMEOUT_LOAD);
-      const uint64_t k_desc = smem_desc_sw128(k_smem, 16, 1024);
-      const uint64_t v_desc = smem_desc_sw128(v_smem, 16, 1024);
-      auto stage_base = [&](int it) { return stage_smem + (it % A_STAGES) * A_STAGE_BYTES; };
-      // S^T = K Q^T and dP^T = V dO^T for queries [64 h, 64 h + 64) of tile `it`: rows 64 h.. of the Q and dO
-      // tiles are 64 x 128 bytes further on (+512 in descriptor units); 16 head-dim elements per MMA = 32 bytes
-      // inside a span, the second span one chunk (16 KiB) further on
-      auto ss_half = [&](int it, int h) {
-        const uint64_t q_desc = smem_desc_sw128(stage_base(it), 16, 1024) + 512 * h;
-        const uint64_t do_desc = q_desc + (TILE_BYTES >> 4);
+      for (int n = 0; ok && n < 2 * n_iter; ++n) {
+        const int it = n >> 1, h = n & 1, s = it % A_STAGES;
+        if (h == 0 && !mbar_wait(q_full(s), (it / A_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) break;
+        if (n > 0 && !mbar_wait(s_free(1 - h), ((n - 1) >> 1) & 1, p.status, WK_ERR_TIMEOUT_P)) break;
+        tc_fence_after();
+        // rows 64 h.. of the Q / dO tile are 64 x 128 bytes further on (+512 in descriptor units); 16 head-dim elements
+        // per MMA = 32 bytes inside a span, the second span one chunk (16 KiB) further on
+        const uint64_t b_desc = smem_desc_sw128(stage_smem + s * A_STAGE_BYTES + which * TILE_BYTES, 16, 1024) + 512 * h;
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint64_t off = (k >> 2) * (CHUNK_BYTES >> 4) + 2 * (k & 3);
-          if (16 * k < DH) mma_f16_ss(st_tmem + HALF_COLS * h, k_desc + off, q_desc + off, idesc_ss, k != 0);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t off = (k >> 2) * (CHUNK_BYTES >> 4) + 2 * (k & 3);
-          if (16 * k < DH) mma_f16_ss(dpt_tmem + HALF_COLS * h, v_desc + off, do_desc + off, idesc_ss, k != 0);
+          if (16 * k < DH) mma_f16_ss(d_tmem, a_desc + off, b_desc + off, idesc, k != 0);
         }
         tc_commit(s_full(h));
-      };
-      // dV += P^T dO and dK += dS^T Q over the same 64 queries.  B operands: the dO / Q tiles again, now read
-      // MN-major (K = queries, 16 per step = 2048 bytes; N = head dim, its two spans 16 KiB apart)
-      auto ts_half = [&](int it, int h) {
-        const uint64_t q_desc = smem_desc_sw128(stage_base(it), CHUNK_BYTES, 1024);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 3) {
+    if (lane == 0 && n_iter > 0) {
+      // dV += P^T dO and dK += dS^T Q over the unit's 64 queries.  B operands: the dO / Q tiles again, now read MN-major
+      // (K = queries, 16 per step = 2048 bytes; N = head dim, its two spans 16 KiB apart)
+      const uint32_t idesc = make_idesc(1, 1, 0, 1, BN, DH);
+      for (int n = 0; n < 2 * n_iter; ++n) {
+        const int it = n >> 1, h = n & 1, s = it % A_STAGES;
+        if (!mbar_wait(q_full(s), (it / A_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) break;
+        if (!mbar_wait(p_full(h), it & 1, p.status, WK_ERR_TIMEOUT_P)) break;
+        tc_fence_after();
+        const uint64_t q_desc = smem_desc_sw128(stage_smem + s * A_STAGE_BYTES, CHUNK_BYTES, 1024) + 512 * h;
         const uint64_t do_desc = q_desc + (TILE_BYTES >> 4);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          // 16 queries = 8 columns; a block of 32 queries keeps its pairs at the start of its own 32 columns
-          mma_f16_ts(tmem_base + A_DV_COL, st_tmem + HALF_COLS * h + 32 * (k >> 1) + 8 * (k & 1),
-                     do_desc + 128 * (4 * h + k), idesc_ts, (it | h | k) != 0);
-        }
+        for (int k = 0; k < 4; ++k)
+          mma_f16_ts(tmem_base + A_DV_COL, tmem_base + A_P_COL + 32 * h + 8 * k, do_desc + 128 * k, idesc, (n | k) != 0);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          mma_f16_ts(tmem_base + A_DK_COL, dpt_tmem + HALF_COLS * h + 32 * (k >> 1) + 8 * (k & 1),
-                     q_desc + 128 * (4 * h + k), idesc_ts, (it | h | k) != 0);
-        }
-      };
-      ok = ok && mbar_wait(q_full(0), 0, p.status, WK_ERR_TIMEOUT_LOAD);
-      if (ok) {
-        tc_fence_after();
-        ss_half(0, 0);
-        ss_half(0, 1);
-      }
-      for (int it = 0; ok && it < n_iter; ++it) {
-        const int s = it % A_STAGES;
-        const bool more = it + 1 < n_iter;
-        if (!mbar_wait(p_full(0), it & 1, p.status, WK_ERR_TIMEOUT_P)) break;
-        tc_fence_after();
-        ts_half(it, 0);
-        if (more) {
-          if (!mbar_wait(q_full((it + 1) % A_STAGES), ((it + 1) / A_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) break;
-          tc_fence_after();
-          ss_half(it + 1, 0);
-        }
-        if (!mbar_wait(p_full(1), it & 1, p.status, WK_ERR_TIMEOUT_P)) break;
-        tc_fence_after();
-        ts_half(it, 1);
-        tc_commit(q_empty(s));
-        if (more) ss_half(it + 1, 1);
-        if (!more) tc_commit(acc_full);
+        for (int k = 0; k < 4; ++k)
+          mma_f16_ts(tmem_base + A_DK_COL, tmem_base + A_DS_COL + 32 * h + 8 * k, q_desc + 128 * k, idesc, (n | k) != 0);
+        tc_commit(p_free(h));
+        if (h == 1) tc_commit(q_empty(s));
+        if (n + 1 == 2 * n_iter) tc_commit(acc_full);
       }
     }
     __syncwarp();
   } else {
     const int quad = warp & 3;
-    const int c = (warp - 2) >> 2;   // which block of 32 of the tile's 128 columns this thread handles
-    const int half = c >> 1;         // the half the block is handed over with
+    const int c = (warp - 4) >> 2;   // which block of 32 of the tile's 128 queries this thread handles
+    const int h = c >> 1;            // its group
     const int r = quad * 32 + lane;  // key row of the tile == TMEM lane
     const int key = n0 + r;
-    const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    // this thread's block: scores in columns [32 c, 32 c + 32) of both buffers
-    const uint32_t st_tmem = tmem_base + lane_addr + A_ST_COL + 32 * c;
-    const uint32_t dpt_tmem = tmem_base + lane_addr + A_DPT_COL + 32 * c;
+    const uint32_t lane_tmem = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     const float beta = p.softmax_scale * LOG2E;
     bool ok = true;
 
+    int m = m_first;  // this iteration's query tile
     for (int it = 0; it < n_iter; ++it) {
-      const int s = it % A_STAGES;
-      const int m0 = (m_first + it % tiles_per_head) * BM;
-      if (!mbar_wait_warp(s_full(half), it & 1, p.status, WK_ERR_TIMEOUT_MMA)) {
+      const int m0 = m * BM;
+      if (++m == num_m) m = m_first;
+      if (!mbar_wait_warp(s_full(h), it & 1, p.status, WK_ERR_TIMEOUT_MMA)) {
         ok = false;
         break;
       }
       tc_fence_after();
+      uint32_t sraw[32], draw[32];
+      tmem_ld32(lane_tmem + A_ST_COL + 32 * (c & 1), sraw);
+      tmem_ld32(lane_tmem + A_DPT_COL + 32 * (c & 1), draw);
+      tc_wait_ld();
+      tc_fence_before();
+      mbar_arrive(s_free(h));
       // the tile's row records: arrays -L and -D of 128 queries each, read four queries at a time
-      const uint32_t stat = stage_smem + s * A_STAGE_BYTES + 2 * TILE_BYTES;
-      // query column c is visible to this key iff key < Nk and (not causal or key <= m0 + c + shift)
-      const int first_col = key >= p.Nk ? BM : (p.causal ? max(0, key - shift - m0) : 0);
-      // uniform over the CTA: does this (key block, query tile) pair contain any masked score?
-      const bool tile_masked = (n0 + BN > p.Nk) || (p.causal && n0 + BN - 1 > m0 + shift);
-      {
-        uint32_t sraw[32], draw[32];
-        tmem_ld32(st_tmem, sraw);
-        tmem_ld32(dpt_tmem, draw);
-        tc_wait_ld();
+      const uint32_t stat = stage_smem + (it % A_STAGES) * A_STAGE_BYTES + 2 * TILE_BYTES + c * 128;
+      uint32_t pw[2][8], dw[2][8];  // P^T and dS^T as bf16 pairs
+      auto elements = [&](auto masked) {
+        // query column i is visible to this key iff key < Nk and (not causal or key <= m0 + 32 c + i + shift)
+        const int first = !decltype(masked)::value ? 0 : key >= p.Nk ? BM : p.causal ? key - shift - m0 - 32 * c : 0;
         const uint64_t beta2 = pack_f32x2(beta, beta);
-        // 16 queries at a time: their bf16 pairs go to the first columns of the block, which its scores have left
 #pragma unroll
-        for (int hq16 = 0; hq16 < 2; ++hq16) {
-          uint32_t pw[8], dw[8];
+        for (int i = 0; i < 8; ++i) {
+          // the same addresses for every thread: shared-memory broadcasts
+          const float4 nl = lds_f4(stat + 16 * i), nd = lds_f4(stat + 512 + 16 * i);
+          const float nlv[4] = {nl.x, nl.y, nl.z, nl.w}, ndv[4] = {nd.x, nd.y, nd.z, nd.w};
 #pragma unroll
-          for (int ii = 0; ii < 4; ++ii) {
-            const int i = 4 * hq16 + ii;
-            // the same addresses for every thread: shared-memory broadcasts
-            const float4 nl = lds_f4(stat + 16 * (c * 8 + i)), nd = lds_f4(stat + 16 * (32 + c * 8 + i));
-            float x0, x1, x2, x3;
-            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sraw[4 * i]), __uint_as_float(sraw[4 * i + 1])), beta2,
-                                   pack_f32x2(nl.x, nl.y)), x0, x1);
-            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sraw[4 * i + 2]), __uint_as_float(sraw[4 * i + 3])), beta2,
-                                   pack_f32x2(nl.z, nl.w)), x2, x3);
-            float p0 = ex2_approx(x0), p1 = ex2_approx(x1), p2 = ex2_approx(x2), p3 = ex2_approx(x3);
-            if (tile_masked) {
-              if (c * 32 + 4 * i + 0 < first_col) p0 = 0.f;
-              if (c * 32 + 4 * i + 1 < first_col) p1 = 0.f;
-              if (c * 32 + 4 * i + 2 < first_col) p2 = 0.f;
-              if (c * 32 + 4 * i + 3 < first_col) p3 = 0.f;
+          for (int x = 0; x < 4; x += 2) {
+            const int e = 4 * i + x;
+            float x0, x1, d0, d1;
+            unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sraw[e]), __uint_as_float(sraw[e + 1])), beta2,
+                                   pack_f32x2(nlv[x], nlv[x + 1])), x0, x1);
+            float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
+            if (decltype(masked)::value) {
+              if (e < first) p0 = 0.f;
+              if (e + 1 < first) p1 = 0.f;
             }
             // dS = P (dP - D)
-            float d0, d1, d2, d3;
             unpack_f32x2(mul_f32x2(pack_f32x2(p0, p1),
-                                   add_f32x2(pack_f32x2(__uint_as_float(draw[4 * i]), __uint_as_float(draw[4 * i + 1])),
-                                             pack_f32x2(nd.x, nd.y))), d0, d1);
-            unpack_f32x2(mul_f32x2(pack_f32x2(p2, p3),
-                                   add_f32x2(pack_f32x2(__uint_as_float(draw[4 * i + 2]), __uint_as_float(draw[4 * i + 3])),
-                                             pack_f32x2(nd.z, nd.w))), d2, d3);
-            pw[2 * ii] = pack_bf16x2(p0, p1);
-            pw[2 * ii + 1] = pack_bf16x2(p2, p3);
-            dw[2 * ii] = pack_bf16x2(d0, d1);
-            dw[2 * ii + 1] = pack_bf16x2(d2, d3);
+                                   add_f32x2(pack_f32x2(__uint_as_float(draw[e]), __uint_as_float(draw[e + 1])),
+                                             pack_f32x2(ndv[x], ndv[x + 1]))), d0, d1);
+            pw[e / 16][e / 2 % 8] = pack_bf16x2(p0, p1);
+            dw[e / 16][e / 2 % 8] = pack_bf16x2(d0, d1);
           }
-          tmem_st8(st_tmem + 8 * hq16, pw);
-          tmem_st8(dpt_tmem + 8 * hq16, dw);
         }
+      };
+      // uniform over the CTA: does this (key block, query tile) pair contain any masked score?
+      if ((n0 + BN > p.Nk) || (p.causal && n0 + BN - 1 > m0 + shift))
+        elements(std::true_type{});
+      else
+        elements(std::false_type{});
+      if (it > 0 && !mbar_wait_warp(p_free(h), (it - 1) & 1, p.status, WK_ERR_TIMEOUT_MMA)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        tmem_st8(lane_tmem + A_P_COL + 16 * c + 8 * i, pw[i]);
+        tmem_st8(lane_tmem + A_DS_COL + 16 * c + 8 * i, dw[i]);
       }
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(p_full(half));
+      mbar_arrive(p_full(h));
     }
 
     if (n_iter > 0 && ok) ok = mbar_wait_warp(acc_full, 0, p.status, WK_ERR_TIMEOUT_MMA);
@@ -434,7 +424,7 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       const int64_t row_off = ((static_cast<int64_t>(b) * p.Hkv + hkv) * p.Nk + key) * DH;
 #pragma unroll 1
       for (int which = 0; which < 2; ++which) {
-        const uint32_t src = tmem_base + lane_addr + (which == 0 ? A_DV_COL : A_DK_COL);
+        const uint32_t src = lane_tmem + (which == 0 ? A_DV_COL : A_DK_COL);
         __nv_bfloat16* dst_row = (which == 0 ? p.dv : p.dk) + row_off;
         const float scale = which == 0 ? 1.f : dk_scale;
 #pragma unroll 1
@@ -475,10 +465,14 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
 // ---------------------------------------------------------------------------
 // 3. dQ
 // ---------------------------------------------------------------------------
-constexpr int B_STAGES = 2;
-constexpr int B_STAGE_BYTES = 2 * TILE_BYTES;  // K tile, V tile
-constexpr int B_SMEM_BYTES = 2 * TILE_BYTES + B_STAGES * B_STAGE_BYTES + 1024 + 256;  // 193 KiB: one CTA per SM
-constexpr int B_S_COL = 0, B_DP_COL = 128, B_DQ_COL = 256;
+// Per tile of 128 keys S and dP are one N = 128 product each (the operands then cost shared memory as many cycles as
+// the tensor pipe; N = 64 half as many again) into one pair of score buffers, which the element-wise warps free as soon as
+// they hold the values in registers; dS goes to columns of its own, of which there are two sets.  So the scores of a tile
+// are under way while dS of the tile before is computed and its product issued.  K has a ring of three tiles and V one of
+// two: V is free once dP is complete, K only after dQ += dS K.
+constexpr int B_K_STAGES = 3, B_V_STAGES = 2;
+constexpr int B_SMEM_BYTES = (2 + B_K_STAGES + B_V_STAGES) * TILE_BYTES + 1024 + 256;  // 225 KiB: one CTA per SM
+constexpr int B_S_COL = 0, B_DP_COL = 128, B_DQ_COL = 256, B_DS_COL = 384;
 
 template <int DH>
 __global__ void __launch_bounds__(THREADS, 1)
@@ -489,16 +483,19 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t q_smem = smem_base;
   const uint32_t do_smem = q_smem + TILE_BYTES;
-  const uint32_t stage_smem = do_smem + TILE_BYTES;
-  const uint32_t bar_base = stage_smem + B_STAGES * B_STAGE_BYTES;
-  const uint32_t q_full = bar_base;
-  auto kv_full = [&](int s) { return bar_base + 8u * (1 + s); };
-  auto kv_empty = [&](int s) { return bar_base + 8u * (1 + B_STAGES + s); };
-  // the two 64-key halves of a tile are handed back and forth separately (h = 0, 1)
-  auto s_full = [&](int h) { return bar_base + 8u * (1 + 2 * B_STAGES + h); };
-  auto p_full = [&](int h) { return bar_base + 8u * (3 + 2 * B_STAGES + h); };
-  const uint32_t acc_full = bar_base + 8u * (5 + 2 * B_STAGES);
-  const uint32_t tmem_slot = acc_full + 8;
+  const uint32_t k_ring = do_smem + TILE_BYTES;
+  const uint32_t v_ring = k_ring + B_K_STAGES * TILE_BYTES;
+  const uint32_t bar_base = v_ring + B_V_STAGES * TILE_BYTES;
+  auto k_full = [&](int s) { return bar_base + 8u * s; };
+  auto k_empty = [&](int s) { return bar_base + 8u * (B_K_STAGES + s); };
+  const uint32_t v_bars = bar_base + 8u * (2 * B_K_STAGES);
+  auto v_full = [&](int s) { return v_bars + 8u * s; };
+  auto v_empty = [&](int s) { return v_bars + 8u * (B_V_STAGES + s); };
+  const uint32_t misc = v_bars + 8u * (2 * B_V_STAGES);
+  const uint32_t q_full = misc, s_full = misc + 8, s_free = misc + 16, acc_full = misc + 24;
+  auto ds_full = [&](int i) { return misc + 32 + 8u * i; };  // the set's dS is in tensor memory
+  auto ds_free = [&](int i) { return misc + 48 + 8u * i; };  // the product that reads it is complete
+  const uint32_t tmem_slot = misc + 64;
 
   const int warp = threadIdx.x / 32;
   const int lane = threadIdx.x % 32;
@@ -517,13 +514,19 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int s = 0; s < B_STAGES; ++s) {
-      mbar_init(kv_full(s), 1);
-      mbar_init(kv_empty(s), 1);
+    for (int s = 0; s < B_K_STAGES; ++s) {
+      mbar_init(k_full(s), 1);
+      mbar_init(k_empty(s), 1);
     }
-    for (int h = 0; h < 2; ++h) {
-      mbar_init(s_full(h), 1);
-      mbar_init(p_full(h), HALF_THREADS);
+    for (int s = 0; s < B_V_STAGES; ++s) {
+      mbar_init(v_full(s), 1);
+      mbar_init(v_empty(s), 1);
+    }
+    mbar_init(s_full, 2);  // S and dP come from two threads
+    mbar_init(s_free, EW_THREADS);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(ds_full(i), EW_THREADS);
+      mbar_init(ds_free(i), 1);
     }
     mbar_init(acc_full, 1);
     mbar_fence_init();
@@ -552,133 +555,123 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         tma_load_4d(do_smem + c * CHUNK_BYTES, &tmap_do, q_full, c * CHUNK, m0, hq, b);
       }
       for (int j = 0; j < n_tiles; ++j) {
-        const int s = j % B_STAGES;
-        const uint32_t ph = (j / B_STAGES) & 1;
-        if (!mbar_wait(kv_empty(s), ph ^ 1, p.status, WK_ERR_TIMEOUT_EMPTY)) break;
-        const uint32_t base = stage_smem + s * B_STAGE_BYTES;
-        mbar_expect_tx(kv_full(s), 2 * chunks * CHUNK_BYTES);
-        for (int c = 0; c < chunks; ++c) {
-          tma_load_4d(base + c * CHUNK_BYTES, &tmap_k, kv_full(s), c * CHUNK, j * BN, hkv, b);
-          tma_load_4d(base + TILE_BYTES + c * CHUNK_BYTES, &tmap_v, kv_full(s), c * CHUNK, j * BN, hkv, b);
-        }
+        const int vs = j % B_V_STAGES, ks = j % B_K_STAGES;
+        if (!mbar_wait(k_empty(ks), ((j / B_K_STAGES) & 1) ^ 1, p.status, WK_ERR_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(k_full(ks), chunks * CHUNK_BYTES);
+        for (int c = 0; c < chunks; ++c)
+          tma_load_4d(k_ring + ks * TILE_BYTES + c * CHUNK_BYTES, &tmap_k, k_full(ks), c * CHUNK, j * BN, hkv, b);
+        if (!mbar_wait(v_empty(vs), ((j / B_V_STAGES) & 1) ^ 1, p.status, WK_ERR_TIMEOUT_EMPTY)) break;
+        mbar_expect_tx(v_full(vs), chunks * CHUNK_BYTES);
+        for (int c = 0; c < chunks; ++c)
+          tma_load_4d(v_ring + vs * TILE_BYTES + c * CHUNK_BYTES, &tmap_v, v_full(vs), c * CHUNK, j * BN, hkv, b);
       }
     }
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (warp == 1 || warp == 2) {
     if (lane == 0 && n_tiles > 0) {
-      // Key tiles are processed as two halves of 64 keys, as in the dK/dV kernel: the tensor pipe works on one
-      // half while the element-wise warps of the other are busy.
-      constexpr uint32_t idesc_ss = make_idesc(1, 1, 0, 0, BM, BN / 2);
-      const uint32_t idesc_ts = make_idesc(1, 1, 0, 1, BM, DH);  // B read MN-major, N = head dimension
-      const uint32_t s_tmem = tmem_base + B_S_COL;
-      const uint32_t dp_tmem = tmem_base + B_DP_COL;
+      // S = Q K^T by warp 1, dP = dO V^T by warp 2, side by side: a thread needs ~90 cycles per MMA it issues here
+      const bool is_s = warp == 1;
+      constexpr uint32_t idesc = make_idesc(1, 1, 0, 0, BM, BN);
+      const uint32_t d_tmem = tmem_base + (is_s ? B_S_COL : B_DP_COL);
+      const uint64_t a_desc = smem_desc_sw128(is_s ? q_smem : do_smem, 16, 1024);
       bool ok = mbar_wait(q_full, 0, p.status, WK_ERR_TIMEOUT_LOAD);
-      const uint64_t q_desc = smem_desc_sw128(q_smem, 16, 1024);
-      const uint64_t do_desc = smem_desc_sw128(do_smem, 16, 1024);
-      auto stage_base = [&](int j) { return stage_smem + (j % B_STAGES) * B_STAGE_BYTES; };
-      // S = Q K^T and dP = dO V^T for keys [64 h, 64 h + 64) of tile j (rows 64 h.. of the K and V tiles: +512 in
-      // descriptor units)
-      auto ss_half = [&](int j, int h) {
-        const uint64_t k_desc = smem_desc_sw128(stage_base(j), 16, 1024) + 512 * h;
-        const uint64_t v_desc = k_desc + (TILE_BYTES >> 4);
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t off = (k >> 2) * (CHUNK_BYTES >> 4) + 2 * (k & 3);
-          if (16 * k < DH) mma_f16_ss(s_tmem + HALF_COLS * h, q_desc + off, k_desc + off, idesc_ss, k != 0);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint64_t off = (k >> 2) * (CHUNK_BYTES >> 4) + 2 * (k & 3);
-          if (16 * k < DH) mma_f16_ss(dp_tmem + HALF_COLS * h, do_desc + off, v_desc + off, idesc_ss, k != 0);
-        }
-        tc_commit(s_full(h));
-      };
-      // dQ += dS K over the same 64 keys: A = dS as bf16 in the dP columns, B = the K tile read MN-major
-      auto ts_half = [&](int j, int h) {
-        const uint64_t k_desc = smem_desc_sw128(stage_base(j), CHUNK_BYTES, 1024);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          // 16 keys = 8 columns; a block of 32 keys keeps its pairs at the start of its own 32 columns
-          mma_f16_ts(tmem_base + B_DQ_COL, dp_tmem + HALF_COLS * h + 32 * (k >> 1) + 8 * (k & 1),
-                     k_desc + 128 * (4 * h + k), idesc_ts, (j | h | k) != 0);
-        }
-      };
-      ok = ok && mbar_wait(kv_full(0), 0, p.status, WK_ERR_TIMEOUT_LOAD);
-      if (ok) {
-        tc_fence_after();
-        ss_half(0, 0);
-        ss_half(0, 1);
-      }
       for (int j = 0; ok && j < n_tiles; ++j) {
-        const int s = j % B_STAGES;
-        const bool more = j + 1 < n_tiles;
-        if (!mbar_wait(p_full(0), j & 1, p.status, WK_ERR_TIMEOUT_P)) break;
+        const int s = is_s ? j % B_K_STAGES : j % B_V_STAGES;
+        const uint32_t full = is_s ? k_full(s) : v_full(s);
+        if (!mbar_wait(full, (is_s ? j / B_K_STAGES : j / B_V_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) break;
+        if (j > 0 && !mbar_wait(s_free, (j - 1) & 1, p.status, WK_ERR_TIMEOUT_P)) break;
         tc_fence_after();
-        ts_half(j, 0);
-        if (more) {
-          if (!mbar_wait(kv_full((j + 1) % B_STAGES), ((j + 1) / B_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) break;
-          tc_fence_after();
-          ss_half(j + 1, 0);
+        const uint64_t b_desc = smem_desc_sw128((is_s ? k_ring : v_ring) + s * TILE_BYTES, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < D / 16; ++k) {
+          const uint64_t off = (k >> 2) * (CHUNK_BYTES >> 4) + 2 * (k & 3);
+          if (16 * k < DH) mma_f16_ss(d_tmem, a_desc + off, b_desc + off, idesc, k != 0);
         }
-        if (!mbar_wait(p_full(1), j & 1, p.status, WK_ERR_TIMEOUT_P)) break;
+        tc_commit(s_full);
+        if (!is_s) tc_commit(v_empty(s));
+      }
+    }
+    __syncwarp();
+  } else if (warp == 3) {
+    if (lane == 0 && n_tiles > 0) {
+      // dQ += dS K: A = dS in tensor memory, B = the K tile read MN-major (16 keys = 2048 bytes, the head dimension's
+      // two spans one chunk apart)
+      const uint32_t idesc = make_idesc(1, 1, 0, 1, BM, DH);
+      for (int j = 0; j < n_tiles; ++j) {
+        const int s = j % B_K_STAGES, set = j & 1;
+        if (!mbar_wait(k_full(s), (j / B_K_STAGES) & 1, p.status, WK_ERR_TIMEOUT_LOAD)) break;
+        if (!mbar_wait(ds_full(set), (j >> 1) & 1, p.status, WK_ERR_TIMEOUT_P)) break;
         tc_fence_after();
-        ts_half(j, 1);
-        tc_commit(kv_empty(s));
-        if (more) ss_half(j + 1, 1);
-        if (!more) tc_commit(acc_full);
+        const uint64_t k_desc = smem_desc_sw128(k_ring + s * TILE_BYTES, CHUNK_BYTES, 1024);
+#pragma unroll
+        for (int k = 0; k < BN / 16; ++k)
+          mma_f16_ts(tmem_base + B_DQ_COL, tmem_base + B_DS_COL + 64 * set + 8 * k, k_desc + 128 * k, idesc, (j | k) != 0);
+        tc_commit(k_empty(s));
+        tc_commit(ds_free(set));
+        if (j + 1 == n_tiles) tc_commit(acc_full);
       }
     }
     __syncwarp();
   } else {
     const int quad = warp & 3;
-    const int c = (warp - 2) >> 2;  // which block of 32 of the tile's 128 columns this thread handles
-    const int half = c >> 1;        // the half the block is handed over with
+    const int c = (warp - 4) >> 2;  // which block of 32 of the tile's 128 columns this thread handles
     const int r = quad * 32 + lane;
     const int row = m0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    // this thread's block: scores in columns [32 c, 32 c + 32) of both buffers
     const uint32_t s_tmem = tmem_base + lane_addr + B_S_COL + 32 * c;
     const uint32_t dp_tmem = tmem_base + lane_addr + B_DP_COL + 32 * c;
+    const uint32_t ds_tmem = tmem_base + lane_addr + B_DS_COL + 16 * c;
     const float beta = p.softmax_scale * LOG2E;
     const float* rec = p.qstat + ((static_cast<int64_t>(b) * p.Hq + hq) * p.nq_pad + m0) * 2 + r;
     const float neg_l = rec[0], neg_d = rec[128];  // -L and -D of this query
-    const int row_limit = min(p.causal ? row + shift : p.Nk - 1, p.Nk - 1);
+    const int row_limit = min(p.causal ? row + shift : p.Nk - 1, p.Nk - 1) - c * 32;
     bool ok = true;
 
     for (int j = 0; j < n_tiles; ++j) {
-      if (!mbar_wait_warp(s_full(half), j & 1, p.status, WK_ERR_TIMEOUT_MMA)) {
+      if (!mbar_wait_warp(s_full, j & 1, p.status, WK_ERR_TIMEOUT_MMA)) {
         ok = false;
         break;
       }
       tc_fence_after();
+      uint32_t sraw[32], draw[32];
+      tmem_ld32(s_tmem, sraw);
+      tmem_ld32(dp_tmem, draw);
+      tc_wait_ld();
+      tc_fence_before();
+      mbar_arrive(s_free);
       const int limit = row_limit - j * BN;  // columns > limit are masked
-      // uniform over the CTA: does this tile contain any masked score?
-      const bool tile_masked = (j * BN + BN > p.Nk) || (p.causal && j * BN + BN - 1 > m0 + shift);
-      {
-        uint32_t sraw[32], draw[32];
-        tmem_ld32(s_tmem, sraw);
-        tmem_ld32(dp_tmem, draw);
-        tc_wait_ld();
-        uint64_t ds[16];  // dS of this query for 32 keys, as packed pairs
-        const uint64_t beta2 = pack_f32x2(beta, beta), nl2 = pack_f32x2(neg_l, neg_l), nd2 = pack_f32x2(neg_d, neg_d);
+      uint64_t ds[16];                       // dS of this query for 32 keys, as packed pairs
+      const uint64_t beta2 = pack_f32x2(beta, beta), nl2 = pack_f32x2(neg_l, neg_l), nd2 = pack_f32x2(neg_d, neg_d);
+      auto elements = [&](auto masked) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float x0, x1;
           unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(sraw[2 * i]), __uint_as_float(sraw[2 * i + 1])), beta2, nl2),
                        x0, x1);
           float p0 = ex2_approx(x0), p1 = ex2_approx(x1);
-          if (tile_masked) {
-            if (c * 32 + 2 * i > limit) p0 = 0.f;
-            if (c * 32 + 2 * i + 1 > limit) p1 = 0.f;
+          if (decltype(masked)::value) {
+            if (2 * i > limit) p0 = 0.f;
+            if (2 * i + 1 > limit) p1 = 0.f;
           }
           ds[i] = mul_f32x2(pack_f32x2(p0, p1),
                             add_f32x2(pack_f32x2(__uint_as_float(draw[2 * i]), __uint_as_float(draw[2 * i + 1])), nd2));
         }
-        store_block_bf16(ds, dp_tmem);
+      };
+      // uniform over the CTA: does this tile contain any masked score?
+      if ((j * BN + BN > p.Nk) || (p.causal && j * BN + BN - 1 > m0 + shift))
+        elements(std::true_type{});
+      else
+        elements(std::false_type{});
+      const int set = j & 1;
+      if (j >= 2 && !mbar_wait_warp(ds_free(set), ((j >> 1) - 1) & 1, p.status, WK_ERR_TIMEOUT_MMA)) {
+        ok = false;
+        break;
       }
+      tc_fence_after();
+      store_block_bf16(ds, ds_tmem + 64 * set);
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(p_full(half));
+      mbar_arrive(ds_full(set));
     }
 
     if (n_tiles > 0 && ok) ok = mbar_wait_warp(acc_full, 0, p.status, WK_ERR_TIMEOUT_MMA);
