@@ -57,7 +57,7 @@ ALL = ["attn_fwd", "gemm_bf16", "attn_bwd", "gemm_mx", "gemm_mx_b", "attn_gqa", 
 # dram__bytes_read.sum + dram__bytes_write.sum per step on one GPU, from ncu captures (attention figures: captured
 # at a fraction of the batch / heads and scaled, traffic grows with batch x heads)
 DRAM_TRAFFIC_BYTES = {
-    # persistent kernel + the two-term launch for the short query blocks (the flag scan moves a few KB)
+    # persistent kernel + the two-term launch for the short query blocks
     "attn_fwd": 2 * (96.5e6 + 31.9e6 + 12.6e6),
     "attn_fwd_small": 96.5e6 + 31.9e6 + 12.6e6,
     "attn_gqa": 4 * (83.2e6 + 85.2e6),
