@@ -939,13 +939,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   auto kv_empty = [&](int s) { return bar_base + 8u * (4 + B_STAGES + s); };
   const uint32_t s_full = bar_base + 8u * (4 + 2 * B_STAGES);  // S and dP of a tile are in TMEM
   const uint32_t s_free = s_full + 8;                          // ... and now in the element-wise threads' registers
-  const uint32_t p_full = s_full + 16;                         // the tile's dS codes and scales are in TMEM
   auto ts_done = [&](int i) { return s_full + 24 + 8u * i; };  // ... and the dQ products have read them (buffer i)
   const uint32_t acc_full = s_full + 40;                       // dQ of the block is complete
   const uint32_t acc_free = s_full + 48;                       // and every element-wise thread has read its part
   auto sched_full = [&](int i) { return acc_free + 8u * (1 + i); };                  // answer i has landed
   auto sched_empty = [&](int i) { return acc_free + 8u * (1 + SCHED_SLOTS + i); };  // and everybody has read it
   const uint32_t tmem_slot = acc_free + 8u * (1 + 2 * SCHED_SLOTS);
+  // The tile's dS codes and scales are in TMEM (buffer i).  One barrier per buffer: the scores of the next tile may be
+  // there before the slowest warp has announced this one, so on a single barrier a fast warp's next arrival could stand in
+  // for that warp's.
+  auto p_full = [&](int i) { return i ? acc_free + 8u * (2 + 2 * SCHED_SLOTS) : s_full + 16; };
   auto sched_resp = [&](int i) { return acc_free + 8u * (4 + 2 * SCHED_SLOTS) + 16u * i; };  // 16-byte answers, 16-byte aligned
 
   const int warp = threadIdx.x / 32;
@@ -968,7 +971,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     }
     mbar_init(s_full, 2);  // S and dP come from two threads
     mbar_init(s_free, EW_THREADS);
-    mbar_init(p_full, EW_THREADS);
+    mbar_init(p_full(0), EW_THREADS);
+    mbar_init(p_full(1), EW_THREADS);
     mbar_init(ts_done(0), 1);
     mbar_init(ts_done(1), 1);
     mbar_init(acc_full, 1);
@@ -1162,7 +1166,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
             break;
           }
           PROBE(17);
-          if (!mbar_wait(p_full, jt & 1, p.status, WK_ERR_TIMEOUT_P)) {
+          if (!mbar_wait(p_full(jt & 1), (jt >> 1) & 1, p.status, WK_ERR_TIMEOUT_P)) {
             ok = false;
             break;
           }
@@ -1273,7 +1277,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
       tmem_st1(sf_tmem + 16 * (jt & 1), sf_d);
       tc_wait_st();
       tc_fence_before();
-      mbar_arrive(p_full);
+      mbar_arrive(p_full(jt & 1));
       PROBE(12);
       PROBE_COUNT(15);
     }
