@@ -359,7 +359,9 @@ def make_attn(dev, world, rank, B, Hq, Hkv, N, d, causal, seed, bf16=False, back
     per_unit = (10.0 if backward else 4.0) * group * N * N * d * (0.5 if causal else 1.0)
     return dict(step=step, e2e_step=lambda: pipe.run(chunks), gather=gather, work=per_unit * B * Hkv,
                 work_local=per_unit * local_units, bound="tensor", dtype="bf16" if bf16 else "fp8",
-                launches=3 * len(launches), h2d=h2d, d2h=d2h, e2e_chunks=len(chunks),
+                # prep, dK/dV, dQ; the FP8 forward's short query blocks (causal) and the others; one kernel else
+                launches=(3 if backward else 2 if causal and not bf16 else 1) * len(launches), h2d=h2d, d2h=d2h,
+                e2e_chunks=len(chunks),
                 gather_bytes=0 if backward else B * Hq * N * d * 2, keep=keep, shard=f"{local_units} of {B * Hkv} (batch, KV head) units")
 
 
@@ -430,7 +432,7 @@ def make_gemm_mx(dev, world, rank, m, n, k, seed, cta_pair=None):
         dsb.copy_(hsb, non_blocking=True)
 
     return dict(step=launch, e2e_step=lambda: pipe.run(chunks, first), gather=lambda: shard.gather_rows(out, m),
-                work=2.0 * m * n * k, work_local=2.0 * (hi - lo) * n * k, bound="tensor", dtype="fp8", launches=3,
+                work=2.0 * m * n * k, work_local=2.0 * (hi - lo) * n * k, bound="tensor", dtype="fp8", launches=2,
                 h2d=h2d, d2h=d2h, e2e_chunks=len(chunks), gather_bytes=m * n * 2, keep=(a8, b8, sa, sb, out),
                 shard=f"rows {lo}:{hi} of {m}", tuned=tuned)
 
