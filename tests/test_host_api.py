@@ -114,3 +114,23 @@ def test_tune_cache_uses_the_reference_file_format(tmp_path, monkeypatch):
     best, results = utils.autotune("fwd", 128, False, 10, 10, 1, [{"a": 1}], lambda cfg: (lambda: None), 1, False) \
         if torch.cuda.is_available() else ({"a": 1}, [])
     assert best == {"a": 1}
+
+
+def test_an_exception_beside_the_released_gil_is_raised():
+    """``_host.launch`` on a device that does not exist: the CUDA error surfaces as ``RuntimeError`` (in a process of its
+    own: without the GIL the interpreter would die of it)."""
+    import subprocess
+    import sys
+
+    code = """
+import ctypes
+from warpy_kernels_b200 import _lib
+entry = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p)(lambda block, stream: 0)
+for call in (lambda h: h.launch(ctypes.cast(entry, ctypes.c_void_p).value, 0, 63), lambda h: h.block_flags(63, 16)):
+    try:
+        call(_lib.host())
+    except RuntimeError:
+        print("raised")
+"""
+    res = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0 and res.stdout.split() == ["raised"] * 2, (res.returncode, res.stderr[-500:])

@@ -142,17 +142,18 @@ at::Tensor empty_strided(at::IntArrayRef sizes, at::IntArrayRef strides, at::Sca
 
 bool aligned(const void* p, uintptr_t n) { return (reinterpret_cast<uintptr_t>(p) & (n - 1)) == 0; }
 
+// Gives up the GIL for as long as it lives; an exception on the way out takes it back too.
+struct GilReleased {
+  PyThreadState* state = PyEval_SaveThread();
+  ~GilReleased() { PyEval_RestoreThread(state); }
+};
+
 // Calls fn(stream) on the current stream of `dev` with that device current and the GIL released.
 template <class F>
 int on_device(int dev, F fn) {
-  int code;
-  Py_BEGIN_ALLOW_THREADS;
-  {
-    const c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(dev)));
-    code = fn(static_cast<void*>(c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev)).stream()));
-  }
-  Py_END_ALLOW_THREADS;
-  return code;
+  const GilReleased gil;
+  const c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(dev)));
+  return fn(static_cast<void*>(c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(dev)).stream()));
 }
 
 // ---- attention --------------------------------------------------------------------------------------------------
@@ -600,10 +601,10 @@ PyObject* bind(PyObject*, PyObject* table) {
 }
 
 // A C++ exception (an allocation that failed, a CUDA error) becomes the Python exception torch raises for it.
-template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t, PyObject*)>
-PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+template <class F>
+PyObject* guard(F call) {
   try {
-    return F(self, args, nargs, kwnames);
+    return call();
   } catch (const c10::OutOfMemoryError& e) {
     PyObject* torch = PyImport_ImportModule("torch");
     PyObject* type = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
@@ -616,14 +617,13 @@ PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObj
   }
   return nullptr;
 }
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t, PyObject*)>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t nargs, PyObject* kwnames) {
+  return guard([&] { return F(self, args, nargs, kwnames); });
+}
 template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
 PyObject* guarded_plain(PyObject* self, PyObject* const* args, Py_ssize_t nargs) {
-  try {
-    return F(self, args, nargs);
-  } catch (const std::exception& e) {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
-  }
-  return nullptr;
+  return guard([&] { return F(self, args, nargs); });
 }
 
 template <auto F>
