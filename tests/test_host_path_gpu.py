@@ -101,3 +101,23 @@ def test_what_is_left_to_python(cuda):
         gemm(a, a[:, :32])
     with pytest.raises(ValueError):
         quantize_mx(a[:, :40])
+
+
+def test_arguments_without_a_value_are_left_to_python(cuda):
+    """An option whose truth value raises, and a whole number beyond a C long: the error of the Python code, not a default."""
+    from warpy_kernels import attn_bwd, attn_fwd, gemm
+
+    q, k, v, scales = _qkv(cuda, True, "bhnd", 128)
+    saved = attn_fwd(q, k, v, *scales)
+    two = torch.tensor([1, 0], device=cuda)
+    for option in ("causal", "return_lse", "lse_natural"):
+        with pytest.raises(RuntimeError, match="ambiguous"):
+            attn_fwd(q, k, v, *scales, **{option: two})
+    with pytest.raises(RuntimeError, match="ambiguous"):
+        attn_bwd(q, k, v, *saved, torch.ones_like(saved[0]), *scales, causal=two)
+    with pytest.raises(ValueError, match="ctas_per_sm"):
+        attn_fwd(q, k, v, *scales, ctas_per_sm=2**70)
+    a = torch.zeros(128, 64, device=cuda, dtype=torch.bfloat16)
+    for option in ("out_mx", "store_pre", "a_trans", "b_trans", "accum", "cta_pair"):
+        with pytest.raises(RuntimeError, match="ambiguous"):
+            gemm(a, a, **{option: two})

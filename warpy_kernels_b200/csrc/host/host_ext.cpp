@@ -105,12 +105,13 @@ struct Params {
     return true;
   }
   bool given(int i) const { return v[i] && v[i] != Py_None; }
-  // A truth value; `fallback` where the argument is absent.
-  bool flag(int i, bool fallback) const {
-    if (!v[i]) return fallback;
-    const int t = PyObject_IsTrue(v[i]);
+  // A truth value, `fallback` where the argument is absent. False if the argument has none (a tensor of several
+  // elements): the Python function asks it again and raises.
+  bool flag(int i, bool fallback, bool& out) const {
+    const int t = v[i] ? PyObject_IsTrue(v[i]) : fallback;
     if (t < 0) PyErr_Clear();
-    return t > 0;
+    out = t > 0;
+    return t >= 0;
   }
 };
 
@@ -245,8 +246,12 @@ PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
     return declined();
   }
   if (!softmax_scale_of(p.v[SCALE], s.d, a.softmax_scale)) return declined();
+  bool with_lse, causal, natural;
+  if (!p.flag(LSE, true, with_lse) || !p.flag(CAUSAL, false, causal) || !p.flag(NATURAL, false, natural))
+    return declined();
   if (p.given(CTAS)) {
     const long n = PyLong_Check(p.v[CTAS]) ? PyLong_AsLong(p.v[CTAS]) : 0;
+    if (n == -1) PyErr_Clear();  // beyond a long
     if (n != 1 && n != 2) return declined();
     a.ctas_per_sm = static_cast<int32_t>(n);
   }
@@ -272,7 +277,6 @@ PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
   a.q = q->data_ptr(), a.k = k->data_ptr(), a.v = v->data_ptr(), a.out = out.data_ptr();
   put_strides(a.q_strides, *q), put_strides(a.k_strides, *k), put_strides(a.v_strides, *v);
   put_strides(a.out_strides, out);
-  const bool with_lse = p.flag(LSE, true);
   at::Tensor lse, pmax;
   if (with_lse) {
     const int64_t nq_pad = (s.Nq + 127) / 128 * 128;  // rows of lse and pmax start every nq_pad entries
@@ -284,7 +288,7 @@ PyObject* attn_fwd(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
     a.write_lse = 1;
   }
   a.B = s.B, a.Hq = s.Hq, a.Hkv = s.Hkv, a.Nq = s.Nq, a.Nk = s.Nk, a.d = s.d;
-  a.causal = p.flag(CAUSAL, false), a.lse_natural = p.flag(NATURAL, false);
+  a.causal = causal, a.lse_natural = natural;
   a.workspace_bytes = abi.attn_fwd_workspace_bytes(a.B, a.Hq, a.Nq);
   void* stream = c10::cuda::getCurrentCUDAStream(s.dev.index()).stream();
   a.workspace = block_flags(s.dev.index(), stream, a.workspace_bytes).data_ptr();
@@ -330,7 +334,8 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
   if (!lse || !pmax || lse->sizes() != at::IntArrayRef(rows) || pmax->sizes() != at::IntArrayRef(rows) ||
       lse->scalar_type() != at::kFloat || lse->device() != s.dev || lse->stride(2) != 1)
     return declined();
-  if (!softmax_scale_of(p.v[SCALE], s.d, a.softmax_scale)) return declined();
+  bool causal;
+  if (!softmax_scale_of(p.v[SCALE], s.d, a.softmax_scale) || !p.flag(CAUSAL, false, causal)) return declined();
   at::Tensor dq = empty({s.B, s.Hq, s.Nq, s.d}, at::kBFloat16, s.dev);
   at::Tensor dk = empty({s.B, s.Hkv, s.Nk, s.d}, at::kBFloat16, s.dev);
   at::Tensor dv = empty({s.B, s.Hkv, s.Nk, s.d}, at::kBFloat16, s.dev);
@@ -343,7 +348,7 @@ PyObject* attn_bwd(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject*
   put_strides(a.out_strides, *out), put_strides(a.dout_strides, *dout);
   a.lse_strides[0] = lse->stride(0), a.lse_strides[1] = lse->stride(1);
   a.B = s.B, a.Hq = s.Hq, a.Hkv = s.Hkv, a.Nq = s.Nq, a.Nk = s.Nk, a.d = s.d;
-  a.causal = p.flag(CAUSAL, false);
+  a.causal = causal;
   const int code = on_device(s.dev.index(), [&](void* st) { return (s.fp8 ? abi.attn_bwd_fp8 : abi.attn_bwd_bf16)(&a, st); });
   if (code) return failed(code, "attn_bwd");
   PyObject* r = PyTuple_New(3);
@@ -403,7 +408,10 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwn
   if (!dev.is_cuda() || b->device() != dev || !device_ok(dev.index())) return declined();
   if (!a->is_contiguous() || !b->is_contiguous() || !aligned(a->data_ptr(), 16) || !aligned(b->data_ptr(), 16))
     return declined();
-  const bool a_trans = p.flag(A_TRANS, false), b_trans = p.flag(B_TRANS, false);
+  bool a_trans, b_trans, store_pre, accum, out_mx, pair;
+  if (!p.flag(A_TRANS, false, a_trans) || !p.flag(B_TRANS, false, b_trans) || !p.flag(STORE_PRE, false, store_pre) ||
+      !p.flag(ACCUM, false, accum) || !p.flag(OUT_MX, false, out_mx) || !p.flag(PAIR, false, pair))
+    return declined();
   const int64_t m = a->size(a_trans ? 1 : 0), k = a->size(a_trans ? 0 : 1);
   const int64_t n = b->size(b_trans ? 1 : 0), kb = b->size(b_trans ? 0 : 1);
   if (kb != k || ((a_trans || b_trans) && fp8) || m < 1 || n < 1 || k < 1) return declined();
@@ -423,7 +431,6 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwn
     else if (PyUnicode_GET_LENGTH(p.v[ACT]) != 0)
       return declined();
   }
-  const bool store_pre = p.flag(STORE_PRE, false), accum = p.flag(ACCUM, false), out_mx = p.flag(OUT_MX, false);
   if ((store_pre && act != 1) || (accum && !p.given(OUT))) return declined();
   at::ScalarType odt = dt;
   at::Tensor out;
@@ -462,7 +469,7 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs, PyObject* kwn
     pre_in = pre->data_ptr();
   }
   int cta_pair = 0;
-  if (p.given(PAIR)) cta_pair = p.flag(PAIR, false) ? 1 : 2;
+  if (p.given(PAIR)) cta_pair = pair ? 1 : 2;
 
   if (!out.defined()) out = empty({m, n}, odt, dev);
   at::Tensor pre_out, q_mx, s_mx, workspace;
