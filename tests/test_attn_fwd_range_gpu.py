@@ -3,9 +3,12 @@
 The tensor-core kernels fix one reference exponent per query row from the row's first 64 keys and can represent
 scores up to 2^100 (69 nats) above it; the reference has no such limit because its reference moves with every key
 tile (``warpy_kernels/attn/fwd_base.py:337-360``).  Query blocks that leave the range are recomputed by the
-library (two-pass fp32 kernel) when the call is given its flag workspace, as the Python wrappers always do.  These
+library in fp32 when the call is given its flag workspace, as the Python wrappers always do.  These
 tests put peaks of 120 to 400 nats behind the first tile and apply the usual gates against the oracle, then check
 the raw C-ABI behaviour without a workspace: the status word says ``WK_ERR_RANGE`` (nothing faults).
+
+Small problems would go to the kernels for few query rows, which hold scores of any range; ``ctas_per_sm`` keeps a call
+on the kernels these tests are about.
 """
 
 import ctypes
@@ -75,7 +78,7 @@ def test_bf16_late_peaks_match_oracle(cuda, causal):
 
     q, k, v = late_peak_qkv(1, 4, 2, 300, 700, 128, [(200, 100.0), (650, 300.0)], seed=2, device=cuda)
     qb, kb, vb = q.bfloat16(), k.bfloat16(), v.bfloat16()
-    out, lse, _ = attn_fwd(qb, kb, vb, causal=causal)
+    out, lse, _ = attn_fwd(qb, kb, vb, causal=causal, ctas_per_sm=2)
     out_ref, lse_ref = R.attention_reference(qb.float().cpu(), kb.float().cpu(), vb.float().cpu(), causal)
     errs = fwd_errors(out, lse, out_ref, lse_ref, 300, 700, causal)
     assert errs["out"] <= 1e-2 and errs["lse"] <= 1e-2, errs  # the reference's bf16 gates (tests/attn/test_fwd.py)
@@ -87,7 +90,7 @@ def test_rows_inside_the_range_are_not_recomputed(cuda):
 
     q, k, v = late_peak_qkv(1, 2, 1, 256, 512, 128, [(300, 60.0)], device=cuda)
     q8, k8, v8, sq, sk, sv = R.quantize_qkv(q, k, v)
-    out, lse, _ = attn_fwd(q8, k8, v8, sq, sk, sv, causal=False)
+    out, lse, _ = attn_fwd(q8, k8, v8, sq, sk, sv, causal=False, ctas_per_sm=2)
     qd, kd, vd = R.dequantize_qkv(q8.cpu(), k8.cpu(), v8.cpu(), sq.cpu(), sk.cpu(), sv.cpu())
     out_ref, lse_ref = R.attention_reference(qd, kd, vd, False)
     gates(fwd_errors(out, lse, out_ref, lse_ref, 256, 512, False))
@@ -122,7 +125,7 @@ def test_without_workspace_the_status_word_reports_the_range(cuda):
     assert lib.wk_status() == 0
     # the same call with the workspace: recomputed, clean status, right answer
     ws = torch.zeros(lib.wk_attn_fwd_workspace_bytes(B, H, Nq), dtype=torch.uint8, device=cuda)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+    a.workspace, a.workspace_bytes, a.ctas_per_sm = ws.data_ptr(), ws.numel(), 2
     assert lib.wk_attn_fwd_fp8(ctypes.byref(a), _lib.stream_ptr(cuda)) == 0
     assert lib.wk_status() == 0 and int(ws.count_nonzero()) == 0
     qd, kd, vd = R.dequantize_qkv(q8.cpu(), k8.cpu(), v8.cpu(), sq.cpu(), sk.cpu(), sv.cpu())
@@ -133,22 +136,59 @@ def test_without_workspace_the_status_word_reports_the_range(cuda):
     assert lib.wk_attn_fwd_fp8(ctypes.byref(a), _lib.stream_ptr(cuda)) == -1
 
 
-@pytest.mark.parametrize("bf16", [False, True])
-def test_head_dim_64_late_peaks_match_oracle(cuda, bf16):
-    """Head dimension 64 takes the same path: flagged blocks are recomputed with half the head-dim lanes idle."""
+@pytest.mark.parametrize("bf16,ctas", [(False, 1), (False, 2), (True, 2)])
+def test_head_dim_64_late_peaks_match_oracle(cuda, bf16, ctas):
+    """Head dimension 64 takes the same path."""
     from warpy_kernels import attn_fwd
 
     q, k, v = late_peak_qkv(1, 4, 2, 300, 700, 64, [(200, 100.0), (650, 300.0)], seed=3, device=cuda)
     if bf16:
         qx, kx, vx = q.bfloat16(), k.bfloat16(), v.bfloat16()
-        out, lse, _ = attn_fwd(qx, kx, vx, causal=True)
+        out, lse, _ = attn_fwd(qx, kx, vx, causal=True, ctas_per_sm=ctas)
         out_ref, lse_ref = R.attention_reference(qx.float().cpu(), kx.float().cpu(), vx.float().cpu(), True)
         errs = fwd_errors(out, lse, out_ref, lse_ref, 300, 700, True)
         assert errs["out"] <= 1e-2 and errs["lse"] <= 1e-2, errs
     else:
         q8, k8, v8, sq, sk, sv = R.quantize_qkv(q, k, v)
-        out, lse, _ = attn_fwd(q8, k8, v8, sq, sk, sv, causal=True)
+        out, lse, _ = attn_fwd(q8, k8, v8, sq, sk, sv, causal=True, ctas_per_sm=ctas)
         qd, kd, vd = R.dequantize_qkv(q8.cpu(), k8.cpu(), v8.cpu(), sq.cpu(), sk.cpu(), sv.cpu())
         out_ref, lse_ref = R.attention_reference(qd, kd, vd, True)
         gates(fwd_errors(out, lse, out_ref, lse_ref, 300, 700, True))
     assert out.shape == q.shape
+
+
+# (B, Hq, Hkv, Nq, Nk, d): more marked blocks than SMs (a CTA of the persistent kernel recomputes several); a ragged last
+# block whose rows partly lie in range; keys that end inside a group of 4 and of 32
+RECOMPUTED = [(2, 8, 2, 1300, 1301, 128), (3, 4, 1, 1155, 1099, 64)]
+
+
+@pytest.mark.parametrize("bf16,ctas", [(False, 1), (False, 2), (True, 2)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("shape", RECOMPUTED)
+def test_recomputed_rows(cuda, shape, causal, bf16, ctas):
+    """Rows beyond the range are as exact as fp32 and a bf16 output allow; sequences of different lengths, one of them
+    without a peak; natural lse; pmax."""
+    from warpy_kernels import attn_fwd
+    from warpy_kernels_b200.attn import fwd_api
+
+    B, Hq, Hkv, Nq, Nk, d = shape
+    q, k, v = late_peak_qkv(B, Hq, Hkv, Nq, Nk, d, [(700, 120.0), (901, 260.0)], seed=5, device=cuda)
+    args = (q.bfloat16(), k.bfloat16(), v.bfloat16()) if bf16 else R.quantize_qkv(q, k, v)
+    deq = tuple(x.float() for x in args) if bf16 else R.dequantize_qkv(*args)
+    used = [Nk, 650, 903][:B]
+    out, lse, pmax = attn_fwd(*args, causal=causal, ctas_per_sm=ctas, lse_natural=True,
+                              seqused_k=torch.tensor(used, dtype=torch.int32, device=cuda))
+    assert int(fwd_api._block_flags(cuda, 16).count_nonzero()) == 0
+    for b, n in enumerate(used):
+        s = deq[0][b] @ deq[1][b, :, :n].repeat_interleave(Hq // Hkv, 0).transpose(-1, -2) / math.sqrt(d)
+        if causal:
+            s = s.masked_fill(torch.arange(n, device=cuda) > torch.arange(Nq, device=cuda)[:, None] + n - Nq, float("-inf"))
+        far = s.amax(-1) - s[..., :64].amax(-1) > 75.0  # 69 nats, and what fp32 logits near 260 may be off
+        assert bool(far.any()) == (n > 700)
+        if n <= 700:
+            continue
+        want = torch.softmax(s.double(), -1) @ deq[2][b, :, :n].repeat_interleave(Hq // Hkv, 0).double()
+        # the output's own rounding to bf16 (2^-9) twice over
+        assert R.rel_l2(out[b][far].double(), want[far]) < 2**-8
+        assert torch.allclose(lse[b][far].double(), torch.logsumexp(s[far].double(), -1), rtol=1e-5)
+        assert torch.allclose(pmax[b][far].double(), torch.softmax(s[far].double(), -1).amax(-1), rtol=2e-3)

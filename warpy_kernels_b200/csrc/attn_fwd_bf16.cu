@@ -49,7 +49,10 @@ constexpr int O_COL = 128;
 constexpr float MAX_BLOCK_EXP = 100.f;  // how far (log2) a block may rise above the row reference
 // After the softmax the first 32 columns of an S buffer hold P: block k of 32 keys keeps its bf16 pairs in
 // columns [16 k, 16 k + 16).
-constexpr int XCH_BYTES = 7 * BM * 4;  // row reference plus (l, lq, m_true) of each group
+constexpr int XCH_BYTES = 7 * BM * 4;  // row reference, then of each group: l, whether the row is computed again (group 0),
+                                       // m_true
+constexpr int X_FAR = 2 * BM * 4;
+static_assert(EXACT_SMEM <= Q_BYTES + 2 * KV_STAGES * KV_BYTES, "the tiles' memory serves the recomputation");
 constexpr int SMEM_BYTES = Q_BYTES + 2 * KV_STAGES * KV_BYTES + XCH_BYTES + 1024 + 256;
 
 struct FwdParams {
@@ -184,6 +187,7 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
 
+  bool again = false;  // this thread's row is out of range and computed again (attn_fwd_exact.cuh)
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
       mbar_expect_tx(q_full, (DH / CHUNK) * Q_CHUNK_BYTES);
@@ -370,10 +374,11 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     // Some key lies more than 2^100 above the first tile's maximum: P has overflowed bf16.
     const bool far = m_true - m_ref > MAX_BLOCK_EXP;
     if (far && !p.exact.flags) atomicCAS(p.status, 0, WK_ERR_RANGE);
-    const bool exact = far && p.exact.flags;
+    again = ok && far && p.exact.flags;
+    if (grp == 0) asm volatile("st.shared.b32 [%0], %1;" ::"r"(x_ref + X_FAR), "r"(again ? 1 : 0) : "memory");
     if (ok) {
       tc_fence_after();
-      const bool empty = !exact && !(l > 0.f);
+      const bool empty = !(l > 0.f);
       const float inv = empty ? 0.f : 1.f / l;
       const int col0 = (DH / 2) * grp;
       __nv_bfloat16* out_row = p.out + b * p.out_stride_b + hq * p.out_stride_h +
@@ -388,12 +393,7 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
-        if (row < p.Nq && exact) {
-          const ExactRow x = exact_row32<true>(p.exact, b, hq, hkv, row, min(row_limit, nk - 1), beta, 1.f, col0 + c * 32,
-                                               out_row + c * 32);
-          m_ref = m_true = x.m;
-          l = x.l;
-        } else if (row < p.Nq) {
+        if (row < p.Nq) {
           uint4* dst = reinterpret_cast<uint4*>(out_row + c * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -405,6 +405,7 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             dst[i] = w;
           }
         }
+        __syncwarp();
       }
       if (p.write_lse && grp == 0 && row < p.Nq) {
         const int64_t off = b * p.lse_stride_b + hq * p.lse_stride_h + row;
@@ -415,12 +416,16 @@ attn_fwd_bf16_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
   }
 
+  __syncwarp();
   tc_fence_before();
-  __syncthreads();
+  const bool any_again = __syncthreads_or(again);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
   }
+  if (any_again && warp < GROUP_THREADS * 2 / 32)  // every tile and product has been used: shared memory is idle
+    exact_block<true, 2 * GROUP_THREADS>(p, b, hq, m_blk, p.softmax_scale * 1.4426950408889634f, 1.f, smem_base,
+                                         xch_smem + X_FAR, threadIdx.x);
 }
 
 }  // namespace

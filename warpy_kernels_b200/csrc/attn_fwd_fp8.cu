@@ -100,7 +100,10 @@ constexpr int SFA_COL = 16;
 constexpr int SFB_COL = 20;
 constexpr int SFA_LO_COL = 24;
 constexpr int RESID_MAX_TILES = 8;   // query blocks that see at most this many key tiles carry the residual term
-constexpr int XCH_BYTES = 7 * BM * 4;  // row reference plus (l, lq, m_true) of each group
+constexpr int XCH_BYTES = 7 * BM * 4;  // row reference, then of each group: l, whether the row is computed again (group 0),
+                                       // m_true
+constexpr int X_FAR = 2 * BM * 4;
+static_assert(EXACT_SMEM <= Q_BYTES + 2 * KV_STAGES * KV_BYTES, "the tiles' memory serves the recomputation");
 constexpr int SMEM_BYTES = Q_BYTES + 2 * KV_STAGES * KV_BYTES + XCH_BYTES + 1024 + 256;
 
 struct FwdParams {
@@ -262,6 +265,7 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
 
+  bool again = false;  // this thread's row is out of range and computed again (attn_fwd_exact.cuh)
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
       mbar_expect_tx(q_full, Q_BYTES);
@@ -458,10 +462,11 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     }
     const bool far = m_true - m_ref > MAX_BLOCK_EXP;  // some key of the row is out of range (attn_fwd_exact.cuh)
     if (far && !p.exact.flags) atomicCAS(p.status, 0, WK_ERR_RANGE);
-    const bool exact = far && p.exact.flags;
+    again = ok && far && p.exact.flags;
+    if (grp == 0) asm volatile("st.shared.b32 [%0], %1;" ::"r"(x_ref + X_FAR), "r"(again ? 1 : 0) : "memory");
     if (ok) {
       tc_fence_after();
-      const bool empty = !exact && !(l > 0.f);
+      const bool empty = !(l > 0.f);
       const float inv = empty ? 0.f : sv / l;
       const int col0 = (DH / 2) * grp;
       __nv_bfloat16* out_row = p.out + b * p.out_stride_b + hq * p.out_stride_h +
@@ -476,12 +481,7 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] = 0;
         }
-        if (row < p.Nq && exact) {
-          const ExactRow x = exact_row32<false>(p.exact, b, hq, hkv, row, min(row_limit, nk - 1), beta, sv, col0 + c * 32,
-                                               out_row + c * 32);
-          m_ref = m_true = x.m;
-          l = x.l;
-        } else if (row < p.Nq) {
+        if (row < p.Nq) {
           uint4* dst = reinterpret_cast<uint4*>(out_row + c * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
@@ -493,6 +493,7 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             dst[i] = w;
           }
         }
+        __syncwarp();
       }
       if (p.write_lse && grp == 0 && row < p.Nq) {
         const int64_t off = b * p.lse_stride_b + hq * p.lse_stride_h + row;
@@ -503,11 +504,18 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     }
   }
 
+  __syncwarp();
   tc_fence_before();
-  __syncthreads();
+  const bool any_again = __syncthreads_or(again);
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+  if (any_again && warp < GROUP_THREADS * 2 / 32) {  // every tile and product has been used: shared memory is idle
+    const int sc = b * p.Hkv + hkv;
+    exact_block<false, 2 * GROUP_THREADS>(p, b, hq, m_blk,
+                                          p.softmax_scale * p.q_descale[sc] * p.k_descale[sc] * 1.4426950408889634f,
+                                          p.v_descale[sc], smem_base, xch_smem + X_FAR, threadIdx.x);
   }
   if (!RESID) pdl_wait();
 }
@@ -594,30 +602,23 @@ __device__ __noinline__ void wide_mark_block(const FwdParams& p, int b, int hq, 
   }
 }
 
-// Recomputes the query blocks this CTA has marked, every softmax thread 32 columns of a row, and takes the marks back.
-__device__ __noinline__ void wide_recompute(const FwdParams& p, int row_in_block, int grp) {
-  const int num_m = (p.Nq + BM - 1) / BM;
+// Recomputes the query blocks this CTA has marked (called by the M_SOFTMAX_THREADS threads `tid` counts) and takes the
+// marks back.
+__device__ __noinline__ void wide_recompute(const FwdParams& p, uint32_t smem, int tid) {
+  const int num_m = (p.Nq + BM - 1) / BM, blocks = p.B * p.Hq * num_m;
   const int cta = 1 + blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  for (int i = 0; i < p.B * p.Hq * num_m; ++i) {
-    if (p.exact.flags[i] != cta) continue;
-    const int row = (i % num_m) * BM + row_in_block, hq = (i / num_m) % p.Hq, b = i / (num_m * p.Hq);
-    const int hkv = hq / (p.Hq / p.Hkv), sc = b * p.Hkv + hkv, col0 = 32 * grp;
-    const int nk = p.seqused_k ? max(0, min(p.Nk, p.seqused_k[b])) : p.Nk;
-    if (row < p.Nq && col0 < p.d) {
-      const float beta = p.softmax_scale * p.q_descale[sc] * p.k_descale[sc] * 1.4426950408889634f;
-      const ExactRow x = exact_row32<false>(
-          p.exact, b, hq, hkv, row, p.causal ? min(row + nk - p.Nq, nk - 1) : nk - 1, beta, p.v_descale[sc], col0,
-          p.out + b * p.out_stride_b + hq * p.out_stride_h + static_cast<int64_t>(row) * p.out_stride_n + col0);
-      if (p.write_lse && grp == 0) {
-        const int64_t off = b * p.lse_stride_b + hq * p.lse_stride_h + row;
-        const bool empty = !(x.l > 0.f);
-        const float lse = empty ? INFINITY : x.m + log2f(x.l);
-        p.lse[off] = p.lse_natural ? lse * 0.6931471805599453f : lse;
-        p.pmax[off] = empty ? 0.f : exp2f(x.m - lse);
-      }
+  for (int first = 0; first < blocks; first += 32) {
+    const int at = first + (tid & 31);
+    uint32_t marked = __ballot_sync(0xffffffffu, at < blocks && p.exact.flags[at] == cta);  // the same in every warp
+    for (; marked; marked &= marked - 1) {
+      const int i = first + __ffs(marked) - 1;
+      const int hq = (i / num_m) % p.Hq, b = i / (num_m * p.Hq), sc = b * p.Hkv + hq / (p.Hq / p.Hkv);
+      exact_block<false, M_SOFTMAX_THREADS>(p, b, hq, i % num_m,
+                                            p.softmax_scale * p.q_descale[sc] * p.k_descale[sc] * 1.4426950408889634f,
+                                            p.v_descale[sc], smem, 0, tid);
+      asm volatile("bar.sync 2, %0;" ::"n"(M_SOFTMAX_THREADS) : "memory");  // every warp has seen the mark
+      if (tid == 0) p.exact.flags[i] = 0;
     }
-    asm volatile("bar.sync 1, 512;" ::: "memory");  // every softmax thread has seen the mark
-    if (row_in_block == 0 && grp == 0) p.exact.flags[i] = 0;
   }
 }
 
@@ -1116,7 +1117,7 @@ attn_fwd_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   if (warp >= 3) {
     uint32_t marked;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(marked) : "r"(sum_meet + M_MARK_OFFSET) : "memory");
-    if (marked) wide_recompute(p, (warp & 3) * 32 + lane, (warp - 3) >> 2);
+    if (marked) wide_recompute(p, smem_base, threadIdx.x - 96);  // shared memory is idle by now
   }
   pdl_wait();  // does not end before the two-term launch, which started before this one, has
 }
