@@ -490,6 +490,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
       p.pmax[off] = empty ? 0.f : exp2f(m_true - lse);
     }
   }
+  __syncwarp();  // lanes leave the loop at different rows; the barrier wants the warp together
   if (p.splits > 1) cluster_sync();  // nobody leaves while its partial results may still be read
 }
 

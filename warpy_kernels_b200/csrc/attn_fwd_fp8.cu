@@ -681,6 +681,7 @@ __device__ __noinline__ bool wide_store_output(const FwdParams& p, uint32_t xch,
     p.lse[off] = p.lse_natural ? lse * 0.6931471805599453f : lse;
     p.pmax[off] = empty ? 0.f : exp2f(m_true - lse);
   }
+  __syncwarp();  // the caller goes on with warp-wide tensor memory loads
   return true;
 }
 

@@ -386,6 +386,7 @@ attn_rows_kernel(const __grid_constant__ RowsParams p, int stages) {
     *reinterpret_cast<float4*>(merged + r * C::O_PITCH + col) = acc;
     if (col == 0) merged[M_OFF + r] = mm, merged[L_OFF + r] = sum, merged[T_OFF + r] = m_true;
   }
+  __syncwarp();
   if (p.splits > 1)
     cluster_sync();
   else
@@ -438,6 +439,7 @@ attn_rows_kernel(const __grid_constant__ RowsParams p, int stages) {
       p.pmax[off] = empty ? 0.f : exp2f(m_true - lse);
     }
   }
+  __syncwarp();  // lanes leave the loop at different rows; the barrier wants the warp together
   if (p.splits > 1) cluster_sync();  // nobody leaves while its partial results may still be read
 }
 
