@@ -235,8 +235,9 @@ typedef struct {
   const int32_t* seqused_k; /* optional [B] int32: keys each batch item attends to (<= Nk) */
   float softmax_scale;
   int32_t ctas_per_sm; /* fp8 forward: 2 = two CTAs per SM with 64-key tiles, 1 = one CTA per SM with 128-key
-                          rounds and four softmax groups (long sequences), 0 = pick by Nk.  The reference's
-                          tuning option of the same name (warpy_kernels/attn/fwd_api.py:196-208) */
+                          rounds and four softmax groups (long sequences), 0 = pick by the sizes; few query rows and
+                          small problems then may go to kernels of their own, for bf16 too.  The
+                          reference's tuning option of the same name (warpy_kernels/attn/fwd_api.py:196-208) */
   void* workspace;     /* optional scratch of wk_attn_fwd_workspace_bytes(B, Hq, Nq) bytes, 4-byte aligned, zeroed;
                           it is left zero, so one buffer can serve every call.  The tensor-core kernels keep one
                           reference exponent per query row, taken from the row's first 64 keys; with a workspace a row

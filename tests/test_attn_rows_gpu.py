@@ -19,7 +19,13 @@ SHAPES = [
     # FP8 from 1024 keys on: products with the packed rows on the N side, 8 or 16 of them
     (1, 1, 1, 1, 1024, 128, False), (2, 8, 1, 1, 1153, 64, False), (3, 9, 3, 3, 1500, 128, True),
     (1, 32, 2, 2, 3333, 64, True), (20, 16, 2, 1, 1280, 128, False), (1, 2, 1, 8, 1031, 128, True),
+    # more than 32 packed rows, ragged, with keys enough to be worth dividing
+    (1, 4, 2, 33, 1500, 128, True), (1, 2, 1, 100, 1900, 64, True), (1, 1, 1, 49, 3100, 128, False),
 ]
+
+# calls within the same limits whose CTAs would crowd the GPU: 128-row tiles with P in two terms, for any number of keys
+CROWDED = [(8, 8, 8, 128, 128, 128), (4, 8, 8, 180, 180, 64), (36, 4, 4, 37, 574, 64), (14, 2, 2, 47, 720, 128),
+           (40, 32, 32, 17, 707, 128), (30, 16, 16, 32, 1100, 64)]
 
 
 def _inputs(cuda, shape, fp8, seed=0):
@@ -101,3 +107,27 @@ def test_late_peaks(cuda, fp8):
     errs = fwd_errors(out, lse, out_ref, lse_ref, 1, 3000, False)
     assert errs["out"] <= 1e-2 and errs["lse"] <= 5e-2, errs  # lse near 400: fp32 logits in base 2
     assert pmax.min().item() > 0.99
+
+
+@pytest.mark.parametrize("layout", ["bhnd", "bnhd"])
+@pytest.mark.parametrize("fp8", [True, False])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("shape", CROWDED)
+def test_crowded_problems(cuda, shape, causal, fp8, layout):
+    """The line between the kernels for few rows and the 128-row tiles costs no precision: the same gates on this side,
+    with lengths per sequence and without."""
+    from warpy_kernels import attn_fwd
+
+    B, Hq, Hkv, Nq, Nk, d = shape
+    args, deq = _inputs(cuda, shape, fp8, seed=9)
+    if layout == "bnhd":
+        args = (*(x.transpose(1, 2).contiguous().transpose(1, 2) for x in args[:3]), *args[3:])
+    used = [Nk if b % 3 else (Nk * (b + 1)) // B for b in range(B)]
+    for lengths in (None, torch.tensor(used, dtype=torch.int32, device=cuda)):
+        out, lse, pmax = attn_fwd(*args, causal=causal, seqused_k=lengths)
+        for b in range(0, B, max(1, B // 4)):
+            n = Nk if lengths is None else used[b]
+            out_ref, lse_ref = R.attention_reference(deq[0][b : b + 1], deq[1][b : b + 1, :, :n], deq[2][b : b + 1, :, :n], causal)
+            _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, Nq, n, causal), fp8)
+        again = attn_fwd(*args, causal=causal, seqused_k=lengths)
+        assert all(torch.equal(x, y) for x, y in zip(again, (out, lse, pmax)))

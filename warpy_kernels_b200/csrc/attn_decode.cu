@@ -494,13 +494,6 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_cons
   if (p.splits > 1) cluster_sync();  // nobody leaves while its partial results may still be read
 }
 
-int decode_splits(const wk_attn_fwd_args* a, int64_t units, int sms) {
-  // two CTAs per SM; at least two tiles for a split
-  int s = 1;
-  while (s < E_MAX_SPLIT && units * s * 2 <= 2 * sms && a->Nk >= 2 * E_KEYS * s * 2) s *= 2;
-  return s;
-}
-
 template <int NR>
 int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, DecodeParams& p, cudaStream_t stream) {
   using C = DecodeCfg<NR>;
@@ -512,6 +505,13 @@ int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, DecodeParams& p,
 }
 
 }  // namespace
+
+int attn_decode_splits(const wk_attn_fwd_args* a, int64_t units, int sms) {
+  // two CTAs per SM; at least two tiles for a split
+  int s = 1;
+  while (s < E_MAX_SPLIT && units * s * 2 <= 2 * sms && a->Nk >= 2 * E_KEYS * s * 2) s *= 2;
+  return s;
+}
 
 int launch_attn_decode(const wk_attn_fwd_args* a, cudaStream_t stream) {
   const int sms = sm_count();
@@ -549,7 +549,7 @@ int launch_attn_decode(const wk_attn_fwd_args* a, cudaStream_t stream) {
   p.softmax_scale = a->softmax_scale;
   const int rows = a->Hq / a->Hkv * a->Nq;
   const int nr = rows <= 8 ? 8 : 16;
-  p.splits = decode_splits(a, static_cast<int64_t>(a->B) * a->Hkv * ((rows + nr - 1) / nr), sms);
+  p.splits = attn_decode_splits(a, static_cast<int64_t>(a->B) * a->Hkv * ((rows + nr - 1) / nr), sms);
   return nr == 8 ? launch_decode<8>(maps[0], maps[1], p, stream) : launch_decode<16>(maps[0], maps[1], p, stream);
 }
 

@@ -453,7 +453,10 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
   if (a->workspace && (a->workspace_bytes < wk_attn_fwd_workspace_bytes(a->B, a->Hq, a->Nq) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
     return WK_E_ARG;
-  if (attn_rows_applies(a, true)) return launch_attn_rows(a, true, static_cast<cudaStream_t>(stream));
+  const int sms = sm_count();
+  if (sms <= 0) return WK_E_CUDA;
+  if (attn_rows_applies(a) && attn_rows_ahead(a, true, sms))
+    return launch_attn_rows(a, true, static_cast<cudaStream_t>(stream));
   int* status = status_word();
   if (!status) return WK_E_CUDA;
 
@@ -506,8 +509,6 @@ extern "C" int wk_attn_fwd_bf16(const wk_attn_fwd_args* a, void* stream) {
                                   : reinterpret_cast<const void*>(attn_fwd_bf16_kernel<128>);
   if (allow_smem(kernel, SMEM_BYTES)) return WK_E_CUDA;
   const int num_m = (a->Nq + BM - 1) / BM;
-  const int sms = sm_count();
-  if (sms <= 0) return WK_E_CUDA;
   // q, out and a share of k and v
   const int64_t head_bytes = 4ll * a->d * (a->Nq + static_cast<int64_t>(a->Nk) * a->Hkv / a->Hq);
   p.band = a->causal ? band_heads(num_m, a->B * a->Hq, head_bytes, sms) : 1;

@@ -39,6 +39,7 @@
 // average out.
 //
 // Tensor-core bound: 4 . B . Hq . Nq . Nk . d flops (half of that when causal).
+#include <limits.h>
 #include <math.h>
 
 #include <type_traits>
@@ -124,6 +125,7 @@ struct FwdParams {
   float softmax_scale;
   int m_first;  // first query block of this launch (the grid covers gridDim.x blocks from here)
   int band;     // heads whose blocks are handed out together (band_heads)
+  int resid_tiles;  // query blocks that see at most this many key tiles carry P in two terms
   int* status;
   int first_in_call;  // no kernel of this call before this one: wait for the stream's earlier work
   ExactInputs exact;  // rows whose scores outgrow the row reference
@@ -181,7 +183,7 @@ __device__ __forceinline__ float block_max(const uint32_t (&s)[32]) {
   return fmaxf(fmaxf(a0, a1), fmaxf(a2, a3));
 }
 
-// RESID: this instantiation handles the query blocks that see at most RESID_MAX_TILES key tiles and carries P
+// RESID: this instantiation handles the query blocks that see at most p.resid_tiles key tiles and carries P
 // as two e4m3 terms; the other instantiation handles all other blocks.  Both are launched on the full grid and
 // a CTA leaves at once when the block is not of its kind.
 template <bool RESID, int DH>
@@ -232,7 +234,7 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
   // The two-term launch comes first in the stream and lets the main launch start beside it; the main launch in
   // turn does not end before the two-term one has (both write parts of the same output).
   if (RESID) pdl_launch_dependents();
-  if ((n_tiles <= RESID_MAX_TILES) != RESID) {
+  if ((n_tiles <= p.resid_tiles) != RESID) {
     if (!RESID) pdl_wait();
     return;
   }
@@ -521,7 +523,7 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Wide variant (query blocks that see more than RESID_MAX_TILES key tiles): one persistent CTA per SM, 608 threads,
+// Wide variant (query blocks that see more than p.resid_tiles key tiles): one persistent CTA per SM, 608 threads,
 // each working through a list of query blocks.
 //
 //   warp 0       TMA producer: Q of a block (two buffers), then its K and V tiles of 128 keys into four-stage rings
@@ -587,7 +589,7 @@ __device__ __forceinline__ bool wide_item(const FwdParams& p, uint32_t x, uint32
   }
   it.n_tiles = n_tiles;
   it.n_rounds = (n_tiles + 1) / 2;  // 128 keys each; the second half of the last one may be all masked
-  return n_tiles > RESID_MAX_TILES;
+  return n_tiles > p.resid_tiles;
 }
 
 // Some key of a row lies more than 2^MAX_BLOCK_EXP above the row reference: the query block is marked in the workspace as
@@ -1160,7 +1162,12 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   if (a->workspace && (a->workspace_bytes < wk_attn_fwd_workspace_bytes(a->B, a->Hq, a->Nq) ||
                        (reinterpret_cast<uintptr_t>(a->workspace) & 3)))
     return WK_E_ARG;
-  if (attn_rows_applies(a, false)) return launch_attn_rows(a, false, static_cast<cudaStream_t>(stream));
+  const int sms = sm_count();
+  if (sms <= 0) return WK_E_CUDA;
+  // Few rows or a small problem: the kernels for those, or the two-term one below for all blocks, whichever is faster, so
+  // that P keeps its seven or more bits on either side of the line between them.
+  const bool few_rows = attn_rows_applies(a);
+  if (few_rows && attn_rows_ahead(a, false, sms)) return launch_attn_rows(a, false, static_cast<cudaStream_t>(stream));
   int* status = status_word();
   if (!status) return WK_E_CUDA;
 
@@ -1233,16 +1240,15 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   // A problem with no more query blocks than SMs has one CTA per SM either way, and then the wide kernel's four softmax
   // groups are ahead from the start (1000 x 1000 x 4 heads 15.5 / 16.5 us against 18.5 / 22.5).
   const int num_m = (a->Nq + BM - 1) / BM;
-  const int sms = sm_count();
-  if (sms <= 0) return WK_E_CUDA;
   const bool few = static_cast<int64_t>(num_m) * a->Hq * a->B <= sms;
   const bool wide = a->ctas_per_sm == 1 || (a->ctas_per_sm == 0 && (a->Nk >= 2048 || few));
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   // Query blocks that see few key tiles run the two-term variant.  The tile count never decreases with the
   // block index, so without per-batch key lengths the two variants get disjoint block ranges; with seqused_k
   // both cover the whole grid and every CTA picks its variant itself.
-  int m_split = 0;
-  if (!a->seqused_k) {
+  p.resid_tiles = few_rows ? INT_MAX : RESID_MAX_TILES;
+  int m_split = few_rows ? num_m : 0;
+  if (!few_rows && !a->seqused_k) {
     const int shift = a->Nk - a->Nq;
     const int all_tiles = (a->Nk + BN - 1) / BN;
     for (int m = 0; m < num_m; ++m) {
@@ -1251,26 +1257,28 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
         const int last_key = (m * BM + BM < a->Nq ? m * BM + BM : a->Nq) - 1 + shift;
         n = last_key < 0 ? 0 : (last_key / BN + 1 < all_tiles ? last_key / BN + 1 : all_tiles);
       }
-      if (n <= RESID_MAX_TILES) m_split = m + 1;
+      if (n <= p.resid_tiles) m_split = m + 1;
     }
   }
-  const int main_first = a->seqused_k ? 0 : m_split;
-  const int resid_count = a->seqused_k ? num_m : m_split;
+  const bool both = a->seqused_k && !few_rows;
+  const int main_first = both ? 0 : m_split;
+  const int resid_count = both ? num_m : m_split;
+  // q, out and a share of k and v
+  const int64_t head_bytes = a->d * (3ll * a->Nq + 2ll * a->Nk * a->Hkv / a->Hq);
+  auto band = [&](int blocks) { return a->causal ? band_heads(blocks, a->B * a->Hq, head_bytes, sms) : 1; };
   // The short blocks first: their CTAs are many and brief, and the main launch, allowed to start while they still
   // run (programmatic stream serialisation), fills the SMs as they leave instead of waiting for the last of them.
   p.first_in_call = 1;
   if (resid_count > 0) {
     p.m_first = 0;
-    p.band = 1;  // blocks of few tiles
+    p.band = few_rows ? band(num_m) : 1;  // else blocks of few tiles
     if (int r = launch_pdl(k_resid, dim3(resid_count, a->Hq, a->B), THREADS, SMEM_BYTES, st, 1, {&tq, &tk, &tv, &p}))
       return r;
     p.first_in_call = 0;
   }
   if (num_m - main_first > 0) {
     p.m_first = main_first;
-    // q, out and a share of k and v
-    const int64_t head_bytes = a->d * (3ll * a->Nq + 2ll * a->Nk * a->Hkv / a->Hq);
-    p.band = a->causal ? band_heads(num_m - main_first, a->B * a->Hq, head_bytes, sms) : 1;
+    p.band = band(num_m - main_first);
     // wide: one CTA per query block in the grid; the CTAs that start take over the blocks of those that have not yet
     if (int r = launch_pdl(wide ? k_wide : k_main, dim3(num_m - main_first, a->Hq, a->B), wide ? M_THREADS : THREADS,
                                 wide ? M_SMEM_BYTES : SMEM_BYTES, st, 1,

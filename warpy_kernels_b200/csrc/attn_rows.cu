@@ -5,9 +5,9 @@
 // new token per sequence 127 of them are padding, each query head of a group reads K and V again, and a block's keys
 // are walked by one CTA alone.  Here the rows of all query heads that share a KV head are packed, 16 to a CTA, and the
 // keys are split over the four warps of a CTA and over the CTAs of a cluster, which combine their partial results in
-// distributed shared memory.  Decoding reads K and V once and is bound by that (16 sequences of 4096-8192 keys, 64 / 8
-// heads, FP8, 202 MB: see the launch rule for what it measures); a small problem is bound by latency, which the split
-// divides.
+// distributed shared memory.  Decoding reads K and V once and is bound by that (16 sequences of 8192 keys, 64 / 8 heads,
+// BF16: 115 us, 4.7 TB/s; FP8 from 1024 keys on is attn_decode.cu's); a small problem is bound by latency, which the
+// split divides (FP8, 1 x 2 heads, 300 x 777, d 64: 7.2 us).
 //
 // Structure: every thread fetches its own operand fragments with cp.async into a ring that only it reads (no barrier
 // in the loop), 16-byte pieces, so that four lanes cover 64 bytes of a K row and eight lanes a whole V row.  The head
@@ -448,7 +448,9 @@ attn_rows_kernel(const __grid_constant__ RowsParams p, int stages) {
 namespace {
 
 constexpr int R_DECODE_KEYS = 1024;  // from here on FP8 decoding goes to attn_decode.cu
-constexpr int R_DECODE_ROWS = 32;  // packed rows up to which the split is chosen to fill the GPU
+// Packed rows up to which the split is chosen to fill the GPU and FP8 goes to attn_decode.cu: two CTAs' worth.  Problems
+// with more rows and more than 2^20 (d 64: 2^22) score elements were not measured here and keep to the 128-row kernels.
+constexpr int R_DECODE_ROWS = 32;
 
 int rows_splits(const wk_attn_fwd_args* a, int sms) {
   const int64_t rows = static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq;
@@ -485,22 +487,74 @@ int launch_rows(RowsParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-bool attn_rows_applies(const wk_attn_fwd_args* a, bool bf16) {
-  (void)bf16;
+namespace {
+
+bool few_rows(int64_t B, int64_t Hq, int64_t Hkv, int64_t Nq, int64_t Nk, int d) {
+  const int64_t rows = Hq / Hkv * Nq, kv = B * Hkv;
+  if (kv > 65535 || rows > 16 * 65535) return false;
+  return rows <= R_DECODE_ROWS || kv * rows * Nk <= (d == 64 ? 1 << 22 : 1 << 20);
+}
+
+bool decodes(const wk_attn_fwd_args* a, bool bf16) {
+  return !bf16 && a->Nk >= R_DECODE_KEYS && static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq <= R_DECODE_ROWS;
+}
+
+}  // namespace
+
+bool attn_rows_applies(const wk_attn_fwd_args* a) {
   // an explicit choice between the tensor-core kernels, or a caller who wants their range reported, gets those
   if (a->ctas_per_sm != 0 || !a->workspace) return false;
-  const int64_t rows = static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq;
-  const int64_t kv = static_cast<int64_t>(a->B) * a->Hkv;
-  if (kv > 65535 || rows > 16 * 65535) return false;
-  if (rows <= R_DECODE_ROWS) return true;
-  // Against the tensor-core kernels with their 128-row tiles (us, FP8): d 64, 600 x 777: 9 / 15, 2048 x 2048 causal
-  // 13 / 22; d 128, 128 x 128 7 / 15, but 1024 x 512 x 2 23 / 15 and 1536 x 640 x 2 20 / 19.
-  return kv * rows * a->Nk <= (a->d == 64 ? 1 << 22 : 1 << 20);
+  return few_rows(a->B, a->Hq, a->Hkv, a->Nq, a->Nk, a->d);
+}
+
+// Every kernel is taken to cost a start, and per CTA a fixed part and a part per step over the keys; two CTAs of an SM
+// take `both` times as long as one alone, and a grid beyond two CTAs per SM as many times longer as it is larger.  The
+// microseconds are fits to 8192 problems inside few_rows()'s limits (1 to 128 sequences, 1 to 32 KV heads, groups of 1 to
+// 16, 1 to 2048 queries, 16 to 16384 keys), half of them within 5 to 10 % (decoding 17 %).  Which side is ahead is mostly a
+// matter of idle SMs and of padding: FP8, d 128, one query for 16 sequences of 8192 keys, 64 / 8 heads 41 us here and 379
+// there, 1 x 2 heads, 300 x 777, d 64 7.2 and 11.6; but 8 x 8 heads, 128 x 128 30.9 and 6.1, 128 x 32 heads, 32 x 1024
+// 534 and 229 (BF16 841 and 344).  By these figures 3 % of the problems go where they take more than 3 % longer than on
+// the other side, at most 1.5 times; by the row limits alone it was 34 % of the BF16 and 46 % of the FP8 problems up to
+// 512 keys, up to 18 times.  Beyond R_DECODE_ROWS the line is drawn as for 256 keys at least, with 0.3 us in favour of this
+// side, so that a batch item mostly attends to its seqused_k keys in the kernel that a call on the truncated tensors gets
+// (whose results are then the same to the bit); that costs 1 us at most, to one problem in eight.
+bool attn_rows_ahead(const wk_attn_fwd_args* a, bool bf16, int sms) {
+  struct Cost {
+    double start, fixed, step, both;
+  };
+  static const Cost kTiles[2][2] = {{{2.3, 2.0, 0.66, 1.7}, {2.5, 2.2, 0.67, 1.7}},   // [bf16][d 128], 64 keys a step
+                                    {{2.5, 1.9, 0.55, 1.7}, {2.7, 2.1, 0.68, 1.7}}};
+  static const Cost kRows[2][2] = {{{2.6, 1.4, 0.81, 1.55}, {2.2, 3.1, 1.41, 1.65}},
+                                   {{3.0, 1.0, 0.70, 1.6}, {2.1, 2.7, 1.19, 1.7}}};
+  static const Cost kDecode[2] = {{2.4, 3.3, 0.87, 1.65}, {2.15, 4.0, 0.93, 1.7}};
+  auto time = [&](const Cost& c, double steps, double ctas) {
+    const double full = ctas / (2.0 * sms);
+    const double crowd = full <= 0.5 ? 1.0 : full <= 1.0 ? 1.0 + (c.both - 1.0) * (2.0 * full - 1.0) : c.both * full;
+    return c.start + (c.fixed + c.step * steps) * crowd;
+  };
+  const bool wide = a->d == 128;
+  const int64_t rows = static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq, kv = static_cast<int64_t>(a->B) * a->Hkv;
+  const int64_t nq = a->Nq, nk = rows > R_DECODE_ROWS && a->Nk < 256 ? 256 : a->Nk;
+  double tiles = static_cast<double>((nk + 63) / 64);
+  if (a->causal) {  // of a block on average: from those of the first block that sees a key to all of them
+    const int64_t first = (nq < 128 ? nq : 128) + nk - nq;
+    tiles = (tiles + (first > 0 ? (first + 63) / 64 : 1)) / 2 * (nk < nq ? static_cast<double>(nk) / nq : 1.0);
+  }
+  const double blocks = static_cast<double>(a->B) * a->Hq * ((nq + 127) / 128);
+  const double there = time(kTiles[bf16][wide], tiles, blocks) + (rows > R_DECODE_ROWS ? 0.3 : 0.0);
+  if (decodes(a, bf16)) {
+    const int64_t units = kv * (rows <= 8 ? 1 : (rows + 15) / 16);
+    const int s = attn_decode_splits(a, units, sms);
+    return time(kDecode[wide], static_cast<double>(((nk + 127) / 128 + s - 1) / s), static_cast<double>(units) * s) <= there;
+  }
+  const int s = rows_splits(a, sms), keys = bf16 ? 16 : 32, shares = R_WARPS * s;
+  const int64_t ctas = kv * ((rows + R_ROWS - 1) / R_ROWS) * s;
+  return time(kRows[bf16][wide], static_cast<double>(((nk + keys - 1) / keys + shares - 1) / shares),
+              static_cast<double>(ctas)) <= there;
 }
 
 int launch_attn_rows(const wk_attn_fwd_args* a, bool bf16, cudaStream_t stream) {
-  if (!bf16 && a->Nk >= R_DECODE_KEYS && static_cast<int64_t>(a->Hq / a->Hkv) * a->Nq <= R_DECODE_ROWS)
-    return launch_attn_decode(a, stream);
+  if (decodes(a, bf16)) return launch_attn_decode(a, stream);
   const int sms = sm_count();
   if (sms <= 0) return WK_E_CUDA;
   RowsParams p = {};
