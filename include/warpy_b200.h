@@ -236,7 +236,7 @@ typedef struct {
   float softmax_scale;
   int32_t ctas_per_sm; /* fp8 forward: 2 = two CTAs per SM with 64-key tiles, 1 = one CTA per SM with 128-key
                           rounds and four softmax groups (long sequences), 0 = pick by the sizes; few query rows and
-                          small problems then may go to kernels of their own, for bf16 too.  The
+                          small problems (wk_attn_fwd_few_rows) then may go to kernels of their own, for bf16 too.  The
                           reference's tuning option of the same name (warpy_kernels/attn/fwd_api.py:196-208) */
   void* workspace;     /* optional scratch of wk_attn_fwd_workspace_bytes(B, Hq, Nq) bytes, 4-byte aligned, zeroed;
                           it is left zero, so one buffer can serve every call.  The tensor-core kernels keep one
@@ -249,6 +249,11 @@ typedef struct {
 } wk_attn_fwd_args;
 
 int64_t wk_attn_fwd_workspace_bytes(int B, int Hq, int Nq);
+
+/* 1 if a call of these sizes that leaves ctas_per_sm at 0 and has a workspace is one of few query rows, or small: the
+ * library then chooses between kernels of its own for such calls and 128-row tiles, with P in at least 7 bits either way.
+ * 0 if it goes to the kernels ctas_per_sm chooses between. */
+int wk_attn_fwd_few_rows(int B, int Hq, int Hkv, int Nq, int Nk, int d);
 int wk_attn_fwd_fp8(const wk_attn_fwd_args* args, void* stream);
 
 /* BF16 attention forward: q, k, v bf16 (element strides multiples of 8), the three descale

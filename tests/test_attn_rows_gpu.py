@@ -131,3 +131,32 @@ def test_crowded_problems(cuda, shape, causal, fp8, layout):
             _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, Nq, n, causal), fp8)
         again = attn_fwd(*args, causal=causal, seqused_k=lengths)
         assert all(torch.equal(x, y) for x, y in zip(again, (out, lse, pmax)))
+
+
+def test_a_tuned_entry_leaves_few_rows_alone(cuda, tmp_path, monkeypatch):
+    """The tuner chooses between the kernels with 128-row tiles, under a key that rounds lengths up to 1024: its entry,
+    here also for each of them in turn, changes nothing for a token per sequence or a small problem of the same bucket,
+    but does apply to the calls it is for."""
+    from warpy_kernels import attn_fwd
+    from warpy_kernels.attn import autotune_attn_fwd, make_attn_fwd
+    from warpy_kernels_b200 import utils
+    from warpy_kernels_b200.attn import fwd_api
+
+    few = [_inputs(cuda, shape, True)[0] for shape in ((4, 8, 2, 1, 3000, 128), (1, 8, 2, 2, 700, 128), (1, 4, 1, 60, 900, 128))]
+    large = _inputs(cuda, (3, 16, 4, 900, 1000, 128), True)[0]
+    monkeypatch.setattr(utils, "TUNE_CACHE_PATH", str(tmp_path / "none.json"))
+    want = [attn_fwd(*args) for args in few]
+    monkeypatch.setattr(utils, "TUNE_CACHE_PATH", str(tmp_path / "tune.json"))
+    best, _ = autotune_attn_fwd(*large[:3], iters=2, verbose=False, q_descale=large[3], k_descale=large[4], v_descale=large[5])
+    entries = utils._entries()
+    assert entries == {utils.tune_key("fwd", 128, False, 900, 1000, 4): best}
+    for ctas in (best["ctas_per_sm"], 1, 2):
+        for nk in (1000, 3000):
+            utils.tune_store(utils.tune_key("fwd", 128, False, 1, nk, 4), {"ctas_per_sm": ctas})
+        assert fwd_api._tuned_ctas_per_sm(*large[:2], False) == ctas
+        for args, (out, lse, pmax) in zip(few, want):
+            for x, y in zip(attn_fwd(*args), (out, lse, pmax)):
+                assert torch.equal(x, y)
+            launch, prepared, _, _ = make_attn_fwd(*args)
+            launch()
+            assert torch.equal(prepared, out)

@@ -66,6 +66,18 @@ def _check_shapes(q, k, v):
         )
 
 
+def _tuned_ctas_per_sm(q, k, causal):
+    """What ``autotune_attn_fwd`` stored for the shape, or ``None``.
+
+    Few query rows and small problems have kernels of their own, which a stored choice between the other two must not
+    switch off: its key rounds lengths up to 1024 and knows nothing of the batch and the head counts.
+    """
+    B, Hq, Nq, d = q.shape
+    if _lib.lib().wk_attn_fwd_few_rows(B, Hq, k.shape[1], Nq, k.shape[2], d) != 0:
+        return None
+    return (tune_lookup(tune_key("fwd", d, causal, Nq, k.shape[2], Hq // k.shape[1])) or {}).get("ctas_per_sm")
+
+
 def make_attn_fwd(
     q,
     k,
@@ -108,7 +120,9 @@ def make_attn_fwd(
         softmax_scale: Scale on the logits, positive. Defaults to ``1 / sqrt(d)``.
         ctas_per_sm: FP8 inputs: 2 runs the kernel with two CTAs per SM and 64-key tiles, 1 the one with a single
             CTA per SM, 128-key rounds and four softmax groups, which is the faster one on long sequences. ``None``
-            takes the tuned value for the shape (``autotune_attn_fwd``), else 1 from 2048 keys on and 2 below.
+            takes the tuned value for the shape (``autotune_attn_fwd``), else 1 from 2048 keys on or where there are no
+            more query blocks than SMs, and 2 otherwise; a call of few query rows or a small one goes to kernels of its
+            own instead, tuned value or not. Giving it keeps a BF16 call off those kernels too.
         num_stages, pipelined, block_n, block_m, warp_rows, tile_local, lpt, tma, warp_spec, split_kv:
             Other tuning options of the reference's SM80-SM120 kernels; accepted and ignored.
         out: Output buffer, ``[B, Hq, Nq, d]`` bf16 with last stride 1 and even other strides. ``None`` allocates one
@@ -193,8 +207,7 @@ def make_attn_fwd(
     args.seqused_k = seq.data_ptr() if seq is not None else None
     args.softmax_scale = float(softmax_scale)
     if ctas_per_sm is None and not bf16:
-        tuned = tune_lookup(tune_key("fwd", d, causal, Nq, Nk, Hq // Hkv))
-        ctas_per_sm = (tuned or {}).get("ctas_per_sm")
+        ctas_per_sm = _tuned_ctas_per_sm(q, k, causal)
     if ctas_per_sm not in (None, 1, 2):
         raise ValueError("ctas_per_sm must be 1 or 2")
     args.ctas_per_sm = int(ctas_per_sm or 0)
@@ -222,8 +235,7 @@ def make_attn_fwd(
 def common_case(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config):
     """The whole call in compiled code, or ``None`` if it needs a copy, is invalid or not plain."""
     if any_tuned() and config.get("ctas_per_sm") is None and q.dtype == torch.float8_e4m3fn and q.dim() == k.dim() == 4:
-        tuned = tune_lookup(tune_key("fwd", q.shape[3], causal, q.shape[2], k.shape[2], q.shape[1] // k.shape[1]))
-        config["ctas_per_sm"] = (tuned or {}).get("ctas_per_sm")
+        config["ctas_per_sm"] = _tuned_ctas_per_sm(q, k, causal)
     return _lib.host().attn_fwd(q, k, v, q_descale, k_descale, v_descale, causal, softmax_scale, **config)
 
 
@@ -245,7 +257,8 @@ def autotune_attn_fwd(q, k, v, candidates=None, iters=20, verbose=True, **kwargs
     """Time candidate configs and store the fastest in the tune cache, as the reference's tuner does.
 
     The FP8 forward has two kernels to choose from (``ctas_per_sm`` 1 and 2, the default candidates); ``make_attn_fwd``
-    looks the winner up when ``ctas_per_sm`` is not given. The cache entry keeps the reference's key format (``fwd`` /
+    looks the winner up when ``ctas_per_sm`` is not given, except for a call of few query rows or a small one, whose own
+    kernels are not among them. The cache entry keeps the reference's key format (``fwd`` /
     ``fwd_bf16``, head dimension, mask, length buckets, GQA ratio, ``sm100``).
 
     Returns:

@@ -587,6 +587,11 @@ int launch_attn_rows(const wk_attn_fwd_args* a, bool bf16, cudaStream_t stream) 
 
 }  // namespace wk
 
+extern "C" int wk_attn_fwd_few_rows(int B, int Hq, int Hkv, int Nq, int Nk, int d) {
+  if (B <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || Nq <= 0 || Nk <= 0 || (d != 64 && d != 128)) return WK_E_ARG;
+  return wk::few_rows(B, Hq, Hkv, Nq, Nk, d);
+}
+
 // One int per block of 128 queries, rounded up to 16 bytes.
 extern "C" int64_t wk_attn_fwd_workspace_bytes(int B, int Hq, int Nq) {
   if (B <= 0 || Hq <= 0 || Nq <= 0) return 0;
