@@ -87,3 +87,26 @@ def test_fp8_backward_order(cuda, shape):
                        *(s[b : b + 1, hkv : hkv + 1].contiguous() for s in scales), causal=True)
         want = (_heads(grads[0], b, hq, group), _heads(grads[1], b, hkv), _heads(grads[2], b, hkv))
         assert all(R.rel_l2(x, w) < 2**-8 for x, w in zip(one, want))
+
+
+# no more query blocks than SMs: below 2048 keys, with a two-term launch beside the main one, and from 2048 keys on
+@pytest.mark.parametrize("shape,causal", [((1, 16, 16, 1100, 1100, 128), True), ((2, 8, 2, 1024, 1300, 64), False),
+                                          ((1, 9, 9, 2048, 2304, 128), True)])
+def test_few_blocks_repeat_to_the_bit(cuda, shape, causal):
+    """With a kernel of another stream on most SMs, so that many CTAs have to wait for one: a block must not go to a
+    running CTA then, whose sums would be in another order."""
+    from warpy_kernels import attn_fwd
+
+    q, k, v = randn_qkv(*shape, device=cuda)
+    q8, k8, v8, *scales = R.quantize_qkv(q, k, v)
+    busy = R.quantize_qkv(*randn_qkv(1, 1, 1, 100 * 128, 16384, 128, device=cuda))  # 100 query blocks
+    side = torch.cuda.Stream()
+    want = attn_fwd(q8, k8, v8, *scales, causal=causal)
+    attn_fwd(*busy)
+    torch.cuda.synchronize()
+    for _ in range(5):
+        with torch.cuda.stream(side):
+            attn_fwd(*busy)
+        got = [attn_fwd(q8, k8, v8, *scales, causal=causal) for _ in range(4)]
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for one in got for a, b in zip(one, want))

@@ -125,6 +125,7 @@ struct FwdParams {
   float softmax_scale;
   int m_first;  // first query block of this launch (the grid covers gridDim.x blocks from here)
   int band;     // heads whose blocks are handed out together (band_heads)
+  int solo;     // every query block gets a CTA of its own: no block changes hands
   int resid_tiles;  // query blocks that see at most this many key tiles carry P in two terms
   int* status;
   int first_in_call;  // no kernel of this call before this one: wait for the stream's earlier work
@@ -545,7 +546,9 @@ attn_fwd_fp8_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 // (clusterlaunchcontrol.try_cancel) and works on that block as well, and so on until none is left: the blocks are
 // handed out one by one in launch order, as they would be to fresh CTAs, without the start-up and the drain of a
 // CTA in between.  Rounds and blocks are counted through the CTA's whole life: every barrier parity below derives
-// from those running counts.
+// from those running counts.  Which group takes which tile of a block derives from them too, and with it the order of
+// its fp32 sums: results repeat to the bit only where no block changes hands.  A grid that fits the SMs gives every block
+// its own CTA (p.solo), also one that has to wait for an SM because other kernels still run.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int M_BN = 128;          // keys per round
 constexpr int M_KV_BYTES = M_BN * D;
@@ -771,6 +774,7 @@ attn_fwd_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
   // Reads the next answer of the launch control: false if no block was left (or the wait gave up: ok is false then).
   // In a warp whose lanes wait together only one of them counts as a reader (`reader`).
   auto next_block = [&](bool together = false, bool reader = true) {
+    if (p.solo) return false;
     const int slot = n_blocks % M_SCHED_SLOTS;
     const uint32_t parity = (n_blocks / M_SCHED_SLOTS) & 1;
     if (!(together ? mbar_wait_warp(sched_full(slot), parity, p.status, WK_ERR_TIMEOUT_LOAD)
@@ -814,6 +818,7 @@ attn_fwd_fp8_wide_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         }
         }
         if (!ok) break;
+        if (p.solo) break;
         // this block's loads are on their way: ask for another block (the MMAs have rounds in hand meanwhile)
         const int slot = n_blocks % M_SCHED_SLOTS;
         if (n_blocks >= M_SCHED_SLOTS &&
@@ -1246,6 +1251,7 @@ extern "C" int wk_attn_fwd_fp8(const wk_attn_fwd_args* a, void* stream) {
   // Query blocks that see few key tiles run the two-term variant.  The tile count never decreases with the
   // block index, so without per-batch key lengths the two variants get disjoint block ranges; with seqused_k
   // both cover the whole grid and every CTA picks its variant itself.
+  p.solo = few;
   p.resid_tiles = few_rows ? INT_MAX : RESID_MAX_TILES;
   int m_split = few_rows ? num_m : 0;
   if (!few_rows && !a->seqused_k) {

@@ -14,6 +14,12 @@ Only when a caller wants one full tensor back is a collective used: ``gather_row
 they are whenever the unit count divides by the world size (else the shards are padded to equal length for the one
 collective).  In both layouts a rank's shard is one contiguous block of the full tensor, so equal shards are
 gathered in place, with nothing staged or copied around the call.
+
+A shard's result is that of the whole problem up to the order of fp32 sums: how a kernel divides keys, K or the tiles of a
+block over CTAs depends on how many there are, and so on the size of the call.  It is the same to the bit where that
+choice is the same for both: the quantiser and the BF16 backward always, the GEMM when its plan does not split K, the
+BF16 forward beyond the small problems, the FP8 forward below 2048 keys when the shard and the whole both have more query
+blocks than the GPU has SMs, or both have not.
 """
 
 import torch
