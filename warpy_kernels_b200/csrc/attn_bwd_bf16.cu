@@ -544,6 +544,8 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  // The dK/dV kernel lets this one start once the prep kernel, whose results both read, has completed: no wait here
+  // (pdl_load).  TMA brings in the caller's tensors only.
   pdl_launch_dependents();
 
   if (warp == 0) {
@@ -623,7 +625,7 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     const uint32_t ds_tmem = tmem_base + lane_addr + B_DS_COL + 16 * c;
     const float beta = p.softmax_scale * LOG2E;
     const float* rec = p.qstat + ((static_cast<int64_t>(b) * p.Hq + hq) * p.nq_pad + m0) * 2 + r;
-    const float neg_l = rec[0], neg_d = rec[128];  // -L and -D of this query
+    const float neg_l = pdl_load(rec), neg_d = pdl_load(rec + 128);  // -L and -D of this query
     const int row_limit = min(p.causal ? row + shift : p.Nk - 1, p.Nk - 1) - c * 32;
     bool ok = true;
 

@@ -999,6 +999,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   // The dK/dV kernel lets this one start once the prep kernel, whose results both read, has completed: no wait here.
   pdl_launch_dependents();
+  if (threadIdx.x == 0) pdl_acquire_async();  // the thread that issues the TMA loads
 
   // The CTA's list of query blocks: its own grid index first, then the indices of CTAs that have not started, handed
   // out by the launch control (common.cuh) one at a time, in launch order (the blocks with the most key tiles
@@ -1219,7 +1220,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_cons
     const float sq = p.q_descale[sc], sk = p.k_descale[sc];
     const float beta = p.softmax_scale * sq * sk * LOG2E;
     const float* rec = p.qstat + ((static_cast<int64_t>(b) * p.Hq + hq) * p.nq_pad + m0) * 2 + r;
-    const float neg_l = rec[0], neg_d = rec[128];  // log2(g) - L and -sum(dO8 . O) of this query
+    const float neg_l = pdl_load(rec), neg_d = pdl_load(rec + 128);  // log2(g) - L and -sum(dO8 . O) of this query
     const float gsv = p.v_descale[sc];  // dP = sv . dP8 in units of g
     const int row_limit = min(p.causal ? row + shift : p.Nk - 1, p.Nk - 1) - key_base;
     if (n_tiles > 0) ++ci;

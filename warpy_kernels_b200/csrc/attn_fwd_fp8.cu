@@ -128,7 +128,8 @@ struct FwdParams {
   int solo;     // every query block gets a CTA of its own: no block changes hands
   int resid_tiles;  // query blocks that see at most this many key tiles carry P in two terms
   int* status;
-  int first_in_call;  // no kernel of this call before this one: wait for the stream's earlier work
+  int first_in_call;  // no kernel of this call before this one: wait for the stream's earlier work (else the one before has
+                      // waited, in every CTA, before it let this one start; both read the caller's tensors only)
   ExactInputs exact;  // rows whose scores outgrow the row reference
 };
 

@@ -142,6 +142,20 @@ __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// For a kernel that runs beside the one before it and reads what kernels before that one wrote.  Every CTA of the one
+// before executes launch_dependents behind its own wait, so the writers have completed, and their writes are performed at
+// device scope, before any CTA of this grid starts.  The wait makes them visible to the grid that waits; here, where
+// waiting would also wait for the kernel beside, nothing must be read that the SM or the async proxy held before: what the
+// kernel two grids back wrote is read with pdl_load (from L2, not L1), and TMA loads of it are ordered behind
+// pdl_acquire_async.  What the caller passed in was complete before that kernel ran, like the input of any kernel.  (That
+// fence costs the thread 0.5 us; before the loads of every CTA of the BF16 dQ kernel, which needs none, it cost 2 x 32 / 8
+// heads, 2048 x 2048 240 -> 244 us.)
+__device__ __forceinline__ void pdl_acquire_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ float pdl_load(const float* p) {
+  float x;
+  asm volatile("ld.relaxed.gpu.global.f32 %0, [%1];" : "=f"(x) : "l"(p) : "memory");
+  return x;
+}
 
 // ---------------------------------------------------------------------------
 // Which block of an attention problem a CTA takes.  Under the causal mask the blocks of a head differ by up to its
