@@ -41,8 +41,9 @@ def _inputs(cuda, shape, fp8, seed=0):
 
 
 def _check(errs, fp8):
-    # P carries at least 11 (FP8) or 8 (BF16) bits here, so the output's own rounding to bf16 is what remains:
-    # the gates of the bf16 forward hold for both
+    # P carries 8 bits for BF16 inputs; for FP8 11 (f16) below 1024 keys and 7 (two e4m3 terms) in the decode kernel and on
+    # the 128-row tiles.  Its rounding errors average out over the keys and the output's own rounding to bf16 is of the same
+    # size: the gates of the bf16 forward hold for both
     assert errs["out"] <= 1e-2 and errs["lse"] <= 1e-2 and errs["max_abs"] <= 2e-2 and errs["cos"] >= 0.999, errs
 
 
@@ -95,7 +96,8 @@ def test_cache_lengths(cuda, fp8, causal, Nk, fill):
 
 @pytest.mark.parametrize("fp8", [True, False])
 def test_late_peaks(cuda, fp8):
-    """Scores hundreds of nats above the first ones: the reference moves, nothing is recomputed."""
+    """Scores hundreds of nats above the first ones: the row reference of a warp moves (BF16), or is the maximum of each
+    split's first tile, which both peaks are in (FP8)."""
     from tests.test_attn_fwd_range_gpu import late_peak_qkv
     from warpy_kernels import attn_fwd
 
@@ -160,3 +162,33 @@ def test_a_tuned_entry_leaves_few_rows_alone(cuda, tmp_path, monkeypatch):
             launch, prepared, _, _ = make_attn_fwd(*args)
             launch()
             assert torch.equal(prepared, out)
+
+
+# (B, Hq, Hkv, Nq, d, causal): 8 and up to 16 packed rows, one and two groups of them, both head dimensions
+SECOND_PASS = [(1, 8, 1, 1, 128, False), (1, 8, 1, 2, 128, True), (1, 8, 1, 1, 64, False), (1, 6, 1, 5, 64, True)]
+
+
+@pytest.mark.parametrize("used", [3000, 2900])
+@pytest.mark.parametrize("shape", SECOND_PASS)
+def test_decode_second_pass(cuda, shape, used):
+    """Peaks 120 nats above the rest in tiles of 128 keys that are not the first of their split (eight splits of three tiles): each
+    of these splits goes through its keys a second time, with the maximum it then knows.  The peaks weigh the same, so a
+    split that gets its second pass wrong shows.  One length ends inside a tile with a peak, before keys and values that
+    must not count."""
+    from tests.test_attn_fwd_range_gpu import late_peak_qkv
+    from warpy_kernels import attn_fwd
+
+    B, Hq, Hkv, Nq, d, causal = shape
+    q, k, v = late_peak_qkv(B, Hq, Hkv, Nq, 3000, d, [(300, 120.0), (2200, 120.0), (2850, 120.0)], device=cuda)
+    args = R.quantize_qkv(q, k, v)
+    deq = R.dequantize_qkv(*args)
+    nan = torch.full_like(args[1][:, :, used:].float(), float("nan")).to(args[1].dtype)
+    args[1][:, :, used:], args[2][:, :, used:] = nan, nan
+    lengths = torch.full((B,), used, dtype=torch.int32, device=cuda)
+    out, lse, pmax = attn_fwd(*args, causal=causal, seqused_k=lengths)
+    out_ref, lse_ref = R.attention_reference(deq[0], deq[1][:, :, :used], deq[2][:, :, :used], causal)
+    errs = fwd_errors(out, lse, out_ref, lse_ref, Nq, used, causal)
+    assert errs["out"] <= 1e-2 and errs["lse"] <= 5e-2, errs  # lse near 170: fp32 logits in base 2
+    assert torch.allclose(pmax, torch.full_like(pmax, 1 / 3), rtol=2e-2)
+    again = attn_fwd(*args, causal=causal, seqused_k=lengths)
+    assert all(torch.equal(x, y) for x, y in zip(again, (out, lse, pmax)))
