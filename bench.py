@@ -58,18 +58,17 @@ ALL = ["attn_fwd", "gemm_bf16", "attn_bwd", "gemm_mx", "gemm_mx_b", "attn_gqa", 
 # at a fraction of the batch / heads and scaled, traffic grows with batch x heads)
 DRAM_TRAFFIC_BYTES = {
     # persistent kernel + the two-term launch for the short query blocks
-    "attn_fwd": 2 * (96.5e6 + 31.9e6 + 12.6e6),
-    "attn_fwd_small": 96.5e6 + 31.9e6 + 12.6e6,
+    "attn_fwd": 2 * (96.6e6 + 27.3e6 + 12.7e6),
+    "attn_fwd_small": 96.6e6 + 27.3e6 + 12.7e6,
     "attn_gqa": 4 * (83.2e6 + 85.2e6),
     "attn_gqa_small": 83.2e6 + 85.2e6,
     # prep + dK/dV + dQ
-    "attn_bwd": 2 * (155.4e6 + 226.7e6 + 177.3e6),
-    "attn_bwd_small": 155.4e6 + 226.7e6 + 177.3e6,
-    "gemm_mx": 292.8e6 + 201.3e6,
-    "gemm_bf16_8k": 1083.5e6 + 127.0e6,
-    "gemm_bf16_8k_pair": 1083.5e6 + 127.0e6,
-    "gemm_bf16_8k_single": 1377.2e6 + 128.6e6,
-    "quant": 234.9e6 + 82.3e6,
+    "attn_bwd": 2 * (155.2e6 + 222.7e6 + 174.2e6),
+    "attn_bwd_small": 155.2e6 + 222.7e6 + 174.2e6,
+    "gemm_mx": 274.2e6 + 203.9e6,
+    "gemm_bf16_8k": 1078.5e6 + 127.8e6,
+    "gemm_bf16_8k_pair": 1078.5e6 + 127.8e6,
+    "quant": 234.9e6 + 68.4e6,
 }
 
 

@@ -238,11 +238,13 @@ typedef struct {
                           rounds and four softmax groups (long sequences), 0 = pick by the sizes; few query rows and
                           small problems (wk_attn_fwd_few_rows) then may go to kernels of their own, for bf16 too.  The
                           reference's tuning option of the same name (warpy_kernels/attn/fwd_api.py:196-208) */
-  void* workspace;     /* optional scratch of wk_attn_fwd_workspace_bytes(B, Hq, Nq) bytes, 4-byte aligned, zeroed;
-                          it is left zero, so one buffer can serve every call.  The tensor-core kernels keep one
-                          reference exponent per query row, taken from the row's first 64 keys; with a workspace a row
-                          in which some later key lies more than 2^100 (69 nats) above it is computed again in fp32
-                          against its exact maximum, which is what the reference's moving tile maximum
+  void* workspace;     /* optional scratch of wk_attn_fwd_workspace_bytes(B, Hq, Nq) bytes, 4-byte aligned.  It must hold
+                          zeros when the call's work starts and holds zeros again when it has completed, so one buffer
+                          can serve the calls that follow one another on a stream; calls that may run at the same time
+                          (other streams, graphs replayed beside them) need buffers of their own.  The tensor-core
+                          kernels keep one reference exponent per query row, taken from the row's first 64 keys; with a
+                          workspace a row in which some later key lies more than 2^100 (69 nats) above it is computed
+                          again in fp32 against its own maximum, which is what the reference's moving tile maximum
                           (warpy_kernels/attn/fwd_base.py:337-360) achieves.  NULL: no recomputation; such an
                           input then leaves WK_ERR_RANGE (110) in the status word and a wrong result. */
   int64_t workspace_bytes;
