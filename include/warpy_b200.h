@@ -98,9 +98,10 @@ typedef struct {
   void* s_mx;
   int32_t a_trans; /* a is stored [K, M] (warpy_kernels/gemm/api.py:103-104, gemm/base.py:127-135) */
   int32_t b_trans; /* b is stored [K, N] */
-  int32_t cta_pair; /* 1: the CTA-pair kernel (tcgen05 cta_group::2, one 256 x 256 tile per two SMs).  2: never pairs.
-                       0: the library's choice (pairs when the 256 x 256 tiles fill the GPU about as well as
-                       128 x 256 ones).  The results are bit-identical either way. */
+  int32_t cta_pair; /* 1: CTA pairs (tcgen05 cta_group::2, one 256 x 256 tile per two SMs).  2: never pairs (tiles of
+                       128 x 128, or 128 x 256 where pairs would have been chosen).  0: the library's choice, by a cycle
+                       model over m, n and k.  The number of ranges K is divided into is the same for all three, and
+                       with it the bits of the result. */
   int32_t group_m;  /* the reference's tuning option of that name (warpy_kernels/gemm/api.py:55, base.py:87-103):
                        output tiles are visited in groups of group_m tile rows that sweep all tile columns, so the
                        CTAs running at the same time share operand rows in L2.  0 = 8.  Any value gives the same bits. */
@@ -145,9 +146,7 @@ typedef struct {
   int32_t out_f16;      /* 0: out / pre buffers are bf16, 1: fp16 */
   void* pre_out;        /* optional [M,N]: the value before the activation (act = 1) */
   const void* pre_in;   /* [M,N] pre-activation values, required for act = 2 */
-  int32_t cta_pair;     /* kernel choice as in wk_gemm16_args: 0 the library's, 1 CTA pairs (tcgen05 cta_group::2, one
-                           256 x 256 tile per two SMs), 2 single CTAs; bit-identical results.  wk_gemm_mxfp8_noalloc
-                           always runs single CTAs. */
+  int32_t cta_pair;     /* as in wk_gemm16_args.  wk_gemm_mxfp8_noalloc always runs single CTAs (2). */
   int32_t a_scale_tiled; /* 1: a_scale_mx is not the row-major [M, K/32] tensor but the output of wk_tile_mx_scales
                             for it (16-byte aligned): the layout the kernels read, made once for scales that do not
                             change from call to call (weights).  0: row-major, re-tiled into the workspace per call. */

@@ -40,7 +40,7 @@ def _inputs(cuda, shape, fp8, seed=0):
     return q8, R.dequantize_qkv(*q8)
 
 
-def _check(errs, fp8):
+def _check(errs):
     # P carries 8 bits for BF16 inputs; for FP8 11 (f16) below 1024 keys and 7 (two e4m3 terms) in the decode kernel and on
     # the 128-row tiles.  Its rounding errors average out over the keys and the output's own rounding to bf16 is of the same
     # size: the gates of the bf16 forward hold for both
@@ -56,7 +56,7 @@ def test_matches_the_oracle(cuda, shape, fp8):
     args, deq = _inputs(cuda, shape, fp8)
     out, lse, pmax = attn_fwd(*args, causal=causal)
     out_ref, lse_ref = R.attention_reference(*deq, causal)
-    _check(fwd_errors(out, lse, out_ref, lse_ref, Nq, Nk, causal), fp8)
+    _check(fwd_errors(out, lse, out_ref, lse_ref, Nq, Nk, causal))
     rep = Hq // Hkv
     s = (deq[0] @ deq[1].repeat_interleave(rep, 1).transpose(-1, -2)) / d**0.5
     if causal:
@@ -91,7 +91,7 @@ def test_cache_lengths(cuda, fp8, causal, Nk, fill):
             assert bool((out[b] == 0).all()) and bool(torch.isinf(lse[b]).all()) and bool((pmax[b] == 0).all())
             continue
         out_ref, lse_ref = R.attention_reference(deq[0][b : b + 1], deq[1][b : b + 1, :, :n], deq[2][b : b + 1, :, :n], causal)
-        _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, 2, n, causal), fp8)
+        _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, 2, n, causal))
 
 
 @pytest.mark.parametrize("fp8", [True, False])
@@ -130,7 +130,7 @@ def test_crowded_problems(cuda, shape, causal, fp8, layout):
         for b in range(0, B, max(1, B // 4)):
             n = Nk if lengths is None else used[b]
             out_ref, lse_ref = R.attention_reference(deq[0][b : b + 1], deq[1][b : b + 1, :, :n], deq[2][b : b + 1, :, :n], causal)
-            _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, Nq, n, causal), fp8)
+            _check(fwd_errors(out[b : b + 1], lse[b : b + 1], out_ref, lse_ref, Nq, n, causal))
         again = attn_fwd(*args, causal=causal, seqused_k=lengths)
         assert all(torch.equal(x, y) for x, y in zip(again, (out, lse, pmax)))
 

@@ -1,8 +1,8 @@
 """Attention forward host API with the reference's call surface (``warpy_kernels/attn/fwd_api.py:141-548``).
 
-Validation, defaults, output layout and return values follow the reference; the SM80-SM120 tuning knobs are
-accepted and ignored because the sm_100a kernel has one fixed configuration (128 queries per CTA, 128-key tiles,
-TMA loads, dedicated load / MMA / softmax warps).
+Validation, defaults, output layout and return values follow the reference.  Of the SM80-SM120 tuning knobs
+``ctas_per_sm`` chooses between the two kernels for FP8 inputs; the others are accepted and ignored: the library picks
+its kernel and how the keys are divided from the sizes.
 """
 
 import ctypes

@@ -40,7 +40,6 @@ constexpr int D = 128;  // largest head dimension; with 64 (the main kernels are
 constexpr int CHUNK = 64;                        // head-dim elements per 128-byte swizzle span
 constexpr int CHUNK_BYTES = 128 * CHUNK * 2;     // 16 KiB: 128 rows x 128 bytes
 constexpr int TILE_BYTES = 2 * CHUNK_BYTES;      // 32 KiB: 128 rows x 256 bytes
-constexpr int SF_BYTES = 512;
 constexpr int THREADS = 640;        // TMA warp, three MMA warps, 16 element-wise warps (four threads per row of a tile)
 constexpr int EW_THREADS = 512;
 constexpr int GROUP_THREADS = 256;  // dK/dV: the element-wise threads of one 64-query half of a tile
@@ -427,7 +426,6 @@ attn_bwd_bf16_dkdv_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         const uint32_t src = lane_tmem + (which == 0 ? A_DV_COL : A_DK_COL);
         __nv_bfloat16* dst_row = (which == 0 ? p.dv : p.dk) + row_off;
         const float scale = which == 0 ? 1.f : dk_scale;
-#pragma unroll 1
         {
           uint32_t v[32];
           if (n_iter > 0) {  // uniform: TMEM loads are warp-wide
@@ -681,7 +679,6 @@ attn_bwd_bf16_dq_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       tc_fence_after();
       const float scale = p.softmax_scale;
       __nv_bfloat16* dst_row = p.dq + ((static_cast<int64_t>(b) * p.Hq + hq) * p.Nq + row) * DH;
-#pragma unroll 1
       {
         uint32_t v[32];
         if (n_tiles > 0) {

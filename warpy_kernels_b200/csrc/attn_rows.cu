@@ -448,8 +448,10 @@ attn_rows_kernel(const __grid_constant__ RowsParams p, int stages) {
 namespace {
 
 constexpr int R_DECODE_KEYS = 1024;  // from here on FP8 decoding goes to attn_decode.cu
-// Packed rows up to which the split is chosen to fill the GPU and FP8 goes to attn_decode.cu: two CTAs' worth.  Problems
-// with more rows and more than 2^20 (d 64: 2^22) score elements were not measured here and keep to the 128-row kernels.
+// Packed rows up to which the split is chosen to fill the GPU and FP8 goes to attn_decode.cu: two CTAs' worth.  Larger
+// problems with more rows keep to the 128-row tiles.  That is right for up to two query heads per KV head (33 to 64 rows,
+// from 512 keys on: tiles 0.61 of the time here for FP8, 0.44 for BF16, medians of 117 and 128 problems) and gives time
+// away where many heads share one: 1.5 and 1.0 times the time here for groups of 4 to 8, 3.8 and 2.3 for groups of 16.
 constexpr int R_DECODE_ROWS = 32;
 
 int rows_splits(const wk_attn_fwd_args* a, int sms) {

@@ -3,8 +3,9 @@
 ``out = a @ b.T * scale_a * scale_b`` for bf16 inputs (tcgen05 ``kind::f16``) and e4m3 inputs (tcgen05
 ``kind::mxf8f6f4`` with ue8m0 scales per 32 elements along K; unit scales when none are given).  The reference's
 SM80-SM120 tuning knobs (``bk, stages, group_m, min_blocks, bn, frag_pipe, tma, warp_spec, persistent,
-setmaxnreg``) are accepted so existing call sites keep working; the sm_100a kernels have one fixed tiling and
-ignore them, except that ``bn`` and ``bk`` still define the divisibility the reference enforces.
+setmaxnreg``) are accepted so existing call sites keep working; the library chooses its tiles and whether K is divided
+over a cluster from the sizes and ignores them, except that ``bn`` and ``bk`` still define the divisibility the reference
+enforces and ``group_m`` the order of the tiles.
 """
 
 import ctypes
@@ -134,10 +135,10 @@ def make_gemm(
             ``out_mx`` writes them. Needs fp8 inputs.
         out_mx: Whether to also write the result as MXFP8: e4m3 values ``[M, N]`` and ``[M, N / 32]`` uint8 ue8m0
             scales computed from the fp32 values before they are rounded to bf16.
-        cta_pair: Not in the reference. ``True`` runs the CTA-pair kernel (``tcgen05`` ``cta_group::2``: two SMs
-            share a 256 x 256 tile). ``False`` never uses pairs. ``None`` leaves the choice to the library: for 16-bit inputs pairs when the
-            256 x 256 tiles fill the GPU about as well as 128 x 256 ones, for fp8 inputs single CTAs. The results
-            are bit-identical either way.
+        cta_pair: Not in the reference. ``True`` runs CTA pairs (``tcgen05`` ``cta_group::2``: two SMs share a
+            256 x 256 tile). ``False`` never uses pairs: 128 x 128 tiles, or 128 x 256 ones where pairs would have been
+            chosen. ``None`` leaves the choice to the library, by a cycle model over the sizes. Into how many ranges K
+            is divided does not depend on this argument, so the results are bit-identical either way.
         b_scale_mx: ``[N, K / 32]`` uint8 ue8m0 scales of ``b``. Not in the reference (which scales only ``a``);
             ``None`` gives the reference's behaviour. ``b`` plays the weights: its scales are re-tiled into the
             kernels' layout once, when the launch is prepared, so ``launch()`` does not see later in-place changes
@@ -309,7 +310,7 @@ def gemm(a, b, out=None, **kwargs):
 
 
 def candidates_for(fp8):
-    """The variants ``autotune_gemm`` times: single CTAs (128 x 256 tiles) or CTA pairs (``tcgen05``
+    """The variants ``autotune_gemm`` times: single CTAs (128 x 128 or 128 x 256 tiles) or CTA pairs (``tcgen05``
     ``cta_group::2``, 256 x 256 tiles over two SMs), each with tile groups of 8 and of 32 rows (``group_m``: few
     rows suit a narrow output, many a wide one), for 16-bit and for fp8 inputs alike.  The counterpart of the
     reference's ``candidates_for`` (``warpy_kernels/gemm/configs.py``), whose knobs tune its SM80-SM120 kernels."""
