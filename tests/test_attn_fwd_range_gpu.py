@@ -192,3 +192,21 @@ def test_recomputed_rows(cuda, shape, causal, bf16, ctas):
         assert R.rel_l2(out[b][far].double(), want[far]) < 2**-8
         assert torch.allclose(lse[b][far].double(), torch.logsumexp(s[far].double(), -1), rtol=1e-5)
         assert torch.allclose(pmax[b][far].double(), torch.softmax(s[far].double(), -1).amax(-1), rtol=2e-3)
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 1, 300, 900, 128), (2, 4, 2, 200, 700, 64)])
+def test_first_scores_overflow_to_minus_infinity(cuda, shape):
+    """The first 100 keys' scores are -inf in fp32, so the row reference is too and every row is computed again: those keys
+    have no weight and the others theirs."""
+    from warpy_kernels import attn_fwd
+
+    B, Hq, Hkv, Nq, Nk, d = shape
+    q, k, v = late_peak_qkv(B, Hq, Hkv, Nq, Nk, d, [], seed=11, device=cuda)
+    k[:, :, 100:] = 0.0
+    q, k = q * 1e20, k.clone()
+    k[:, :, :100] = -1e20  # q . k about -1e42
+    out, lse, pmax = attn_fwd(q.bfloat16(), k.bfloat16(), v.bfloat16(), ctas_per_sm=2)
+    want = v.bfloat16().double()[:, :, 100:].mean(2).repeat_interleave(Hq // Hkv, 1)[:, :, None].expand(out.shape)
+    assert R.rel_l2(out.double(), want) < 2**-8
+    assert torch.allclose(lse, torch.full_like(lse, math.log2(Nk - 100)), rtol=1e-5)
+    assert torch.allclose(pmax, torch.full_like(pmax, 1 / (Nk - 100)), rtol=1e-4)

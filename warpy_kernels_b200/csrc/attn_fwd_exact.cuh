@@ -180,9 +180,10 @@ __device__ __noinline__ void exact_block(const Params& p, int b, int hq, int m_b
 #pragma unroll
             for (int i = 0; i < 16; ++i) o[h][i] *= f;
           }
+          const float ref = m[h] > -INFINITY ? m[h] : 0.f;  // the scores so far may all have overflowed to -inf
 #pragma unroll
           for (int u = 0; u < 4; ++u) {  // a masked key has no part in the row, whatever its V holds
-            s[h][u] = c0 + j + u <= limit[h] ? exp2f(s[h][u] - m[h]) : 0.f;
+            s[h][u] = c0 + j + u <= limit[h] ? exp2f(s[h][u] - ref) : 0.f;
             l[h] += s[h][u];
           }
         }
